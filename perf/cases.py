@@ -21,7 +21,7 @@ import sys
 
 import torch
 
-sys.path.insert(0, os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "pytorch-window-matmul_b200"))
+sys.path.insert(0, os.path.abspath("pytorch-window-matmul_b200"))   # (the working folder is the root of the repository)
 from window_matmul import unwindow_matmul, window_matmul, window_softmax  # noqa: E402
 
 _DTYPES = {"float32": torch.float32, "float16": torch.float16, "bfloat16": torch.bfloat16}
@@ -164,4 +164,8 @@ def work(case):
 
 
 def tolerance(case):
-    return {"rel": 1e-5} if case["dtype"] == "float32" and not case["autocast"] else {"rel": 1e-2}
+    # Measured against the same pass in float64: bfloat16 up to 4.9e-3, float16 up to 6.1e-4 (both: the rounded bands between
+    # the operators), float32 up to 5.2e-7 (sums of up to 1025 terms)
+    if case["dtype"] == "float16" or case["autocast"]:
+        return {"rel": 2.5e-3}
+    return {"rel": 5e-6} if case["dtype"] == "float32" else {"rel": 1e-2}
