@@ -264,8 +264,14 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return y;
 }
 
+// Row lengths are rounded up to one of these numbers of elements per lane: a variant serves rows longer than 32 times the
+// next smaller number (launch_ring picks the first that fits), so that many steps exist for every lane of every row.
+constexpr int ring_steps_in_every_row(int epl) {
+  return epl <= 2 ? 1 : epl <= 3 ? 2 : epl <= 5 ? 3 : epl <= 9 ? 5 : epl <= 13 ? 9 : epl <= 17 ? 13 : epl <= 25 ? 17 : 25;
+}
+
 // NR rows at once (independent instruction streams for the scheduler).  prow[n] / grow[n]: the rows in shared memory;
-// full[n]: every slot of the row is live, so only the last element of a lane needs a bound check.
+// full rows: every slot is live, so only the last steps of a lane need a bound check.
 template <typename T, int EPL, int NR, bool BWD, bool PER_THREAD>
 __device__ __forceinline__ void ring_rows(T *const (&prow)[NR], T *const (&grow)[NR], int W, const int (&jlo)[NR],
                                           const unsigned (&width)[NR], float scale, int lane) {
@@ -275,8 +281,8 @@ __device__ __forceinline__ void ring_rows(T *const (&prow)[NR], T *const (&grow)
   bool all_full = true;
 #pragma unroll
   for (int n = 0; n < NR; ++n) all_full = all_full && jlo[n] == 0 && width[n] == (unsigned)W;
-  // elements below `safe` exist for every lane whatever the row (warp-per-row: all but the last step)
-  constexpr int SAFE = PER_THREAD ? 0 : EPL - 1;
+  // steps below SAFE exist for every lane whatever the row
+  constexpr int SAFE = PER_THREAD ? 0 : ring_steps_in_every_row(EPL);
   if constexpr (!BWD) {
     const float c = scale * kLog2e;
     float x[NR][EPL];

@@ -74,6 +74,15 @@ def test_band_softmax_forward_backward(sm, shape, dtype, mask):
     assert (np.abs(g - want_g) <= bound).all(), "gradient: worst %.2f" % (np.abs(g - want_g) / bound).max()
 
 
+# Rows whose length is rounded up to a compiled number of elements per lane (7 -> 9, 10 -> 13, 14 -> 17, 19 -> 25, 26 -> 33
+# per lane), many enough for the ring kernel: a lane must not touch the elements past its row's end, which are the next
+# row's (or lie past the stage).
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape", [(2, 400, 50), (2, 500, 100), (1, 900, 150), (1, 1000, 220), (1, 1300, 300), (3, 64, 414), (1, 1100, 414)])
+def test_row_lengths_between_the_compiled_ones(sm, shape, dtype):
+    test_band_softmax_forward_backward(sm, shape, dtype, True)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_band_softmax_in_place_and_poisoned_padding(sm, dtype):
     """In place, and with NaN stored in the out-of-sequence slots of the scores and of the incoming gradient: the masked
