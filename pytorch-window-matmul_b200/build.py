@@ -15,7 +15,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "window_matmul", "libwmm_b200.so")
-SOURCES = ["wmm_api.cu", "wmm_generic.cu", "wmm_tc.cu", "wmm_small.cu", "wmm_softmax.cu", "wmm_halo.cu"]
+SOURCES = ["wmm_api.cu", "wmm_generic.cu", "wmm_exact32.cu", "wmm_tc.cu", "wmm_small.cu", "wmm_softmax.cu", "wmm_halo.cu"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -60,7 +60,7 @@ def build(force=False, verbose=False, defines=(), out=None):
         if r.returncode:
             raise RuntimeError("nvcc failed on " + cmd[-3])
 
-    with ThreadPoolExecutor(max_workers=4) as ex:
+    with ThreadPoolExecutor(max_workers=8) as ex:
         list(ex.map(run, jobs))
     objs = [os.path.join(obj_dir, s[:-3] + ".o") for s in SOURCES]
     if force or jobs or _stale(lib, objs):

@@ -36,6 +36,8 @@ enum Primitive { BAND_NT = 1, BAND_N = 2, BAND_T = 3 };
 
 // Launchers.  Each returns cudaSuccess or the launch error; `launches` is incremented per kernel.
 cudaError_t launch_generic(Primitive prim, const Problem &p, cudaStream_t stream, int *launches);
+// fp32 with fused multiply-adds in exact order (the part of the CUDA-core family that fp32 takes without split rounding).
+cudaError_t launch_exact32(Primitive prim, const Problem &p, cudaStream_t stream);
 
 // Tensor-core (tcgen05) family: `eligible` is a pure host-side predicate on shape, dtype, strides and
 // alignment; `launch_tensor` must only be called when it holds.

@@ -1,0 +1,425 @@
+// fp32 in exact order on the CUDA cores: each output element is ONE chain of fused multiply-adds over the ascending
+// reduction index (the order and rounding of the reference's kernels, csrc/window_matmul/cuda/window_matmul_cuda.cu:24-35,
+// 64-83), no split-K and no partial sums.  Any shape, any strides.
+//
+// All three primitives are the register-tiled product C[TM x TN] += A[TM x 16] B[16 x TN] in dense coordinates:
+//   band_nt  C(i, p) = sum_h X[i,h] Y[p,h]        stored at Band[i, p - off - i + w]
+//   band_n   C(i, h) = sum_p Band[i, p-off-i+w] Y[p,h]
+//   band_t   C(p, h) = sum_i Band[i, p-off-i+w] X[i,h]
+// What bounds them is the FFMA pipe, so the loop is built to keep nothing else in its way:
+//   * fma.rn.f32x2: one instruction is two independent chains (two neighbouring columns), each rounded as a scalar fmaf, for
+//     the pipe time of two but one issue slot.  The free slots take the shared-memory reads and the swapped pairs.
+//   * a CTA is ONE warp with its own tile and its own staging: no barrier anywhere, and a warp leaves out the slices its rows
+//     do not touch without holding up others (at w = 256: 544 reduction steps instead of 640 for a tile of 128 rows).
+//   * slices of 16 reduction steps come through cp.async (4 bytes an element, so any stride and any odd band row goes
+//     straight to its place in shared memory; 16 bytes where an operand row allows it), one slice ahead; what lies outside
+//     the band or the sequence is zero-filled by the copy.  Whole slices inside the band take no checks.
+//   * slices outside the sequence are never walked: a window wider than the sequence costs what the sequence does.
+// With finite operands a zero term leaves a sum unchanged (up to the sign of a zero sum).
+// Measured (B200, B=96, M=4096, N=64, w=256, one launch; before = 128 x 64 tiles by CTAs of 256 threads, scalar fmaf and
+// register-staged loads): band_n 950 -> 570 us, band_t 966 -> 562 us, band_nt 957 -> 786 us: 46 / 46 / 33 TFLOP/s of band
+// work (50 with the edges of the tiles).  A loop of nothing but these instructions reaches 63.7, of scalar fmaf 51.
+// band_nt writes 32 x 64 outputs per 64 reduction steps, which is what it spends the rest on.
+#include "wmm_common.cuh"
+
+namespace wmm {
+
+namespace {
+
+constexpr int XK = 16;          // reduction steps per slice
+constexpr int XTHREADS = 32;    // one warp, 4 (rows) x 8 (columns) threads
+
+__device__ __forceinline__ uint32_t xsmem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void cp4(uint32_t dst, const float *src, bool ok) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(ok ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void cp16(uint32_t dst, const float *src, bool ok) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+// two floats as the operand of fma.rn.f32x2
+__device__ __forceinline__ uint64_t pair(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void fma2(uint64_t &d, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float2 halves(uint64_t v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+
+struct ExactParams {
+  const float *a, *b;
+  float *o;
+  int64_t a_sb, a_sr, a_sc, b_sb, b_sr, b_sc, o_sb, o_sr, o_sc;
+  int M, N, w, Mo, off, lo, hi, nrt, nct, cspan;   // cspan (band_nt): column tiles a warp takes one after another
+  int vec_b, vec_o;   // 16-byte accesses along the hidden index are aligned
+};
+
+// MR x MC outputs per thread; a tile is 4*MR rows x 8*MC columns.
+// BKF: the reduction index is the fastest-varying one of the B operand (picks which index neighbouring threads walk).
+template <int PRIM, int MR, int MC, bool BKF>
+__global__ void __launch_bounds__(XTHREADS, 12) band_exact32_kernel(const ExactParams p) {
+  constexpr int TM = 4 * MR, TN = 8 * MC;
+  constexpr bool AKF = PRIM != BAND_T;                   // the reduction index is the fastest-varying one of A in memory
+  constexpr int AP = TM + 4, A_FLOATS = XK * AP;         // pitch of the [k][m] tile
+  constexpr int BP = TN + 4;                             // pitch of the [k][n] tile
+  constexpr int STAGE = A_FLOATS + XK * BP;
+  // Slices ahead: one where a slice is long work and twelve warps share an SM, three for the smallest tiles, whose slice
+  // takes less time than its successor's way from memory.
+  constexpr int STAGES = MR >= 4 ? 2 : 4;
+  constexpr int OUT_P = 36;                              // band_nt: TM rows of 32 columns on their way out
+  static_assert(PRIM != BAND_NT || TM * OUT_P <= STAGE, "the outgoing half tile lies in a staging buffer");
+  __shared__ __align__(16) float smem[STAGES * STAGE];
+
+  int b, rt, cg;
+  {
+    unsigned lin = blockIdx.x;
+    cg = (int)(lin % (unsigned)p.nct);
+    lin /= (unsigned)p.nct;
+    rt = (int)(lin % (unsigned)p.nrt);
+    b = (int)(lin / (unsigned)p.nrt);
+  }
+  const int lane = threadIdx.x;
+  const int ty = lane >> 3, tx = lane & 7;
+  const int W = 2 * p.w + 1;
+  const int r0 = rt * TM;
+  // Rows and columns of a thread: groups of four (or two) neighbours, each read with one 16-byte (8-byte) access.
+  auto row_of = [&](int u) -> int { return MR >= 4 ? (u >> 2) * 16 + ty * 4 + (u & 3) : ty * MR + u; };
+  auto col_of = [&](int v) -> int { return (v >> 2) * 32 + tx * 4 + (v & 3); };
+
+  // The operands in tile coordinates: A(m, k) at a0 + m * a_m + k * a_k, valid for max(klo, m) <= k < min(khi, m + W) on band
+  // operands, klo <= k < khi on others, and m_lo <= m < m_hi; B(k, n) at b0 + k * b_k + n * b_n, klo <= k < khi, n_lo <= n < n_hi.
+  const float *a0, *b0;
+  int64_t a_m, a_k, b_k, b_n;
+  int klo, khi, m_lo = 0, m_hi, n_lo = 0, n_hi, c0;
+  int ctiles = 1;                                        // column tiles of this warp
+  if (PRIM == BAND_NT) {
+    c0 = cg * p.cspan * TN;
+    const int pos0 = r0 - p.w + p.off + c0;              // position of column 0
+    a0 = p.a + (int64_t)b * p.a_sb + (int64_t)r0 * p.a_sr;
+    a_m = p.a_sr; a_k = p.a_sc;
+    b0 = p.b + (int64_t)b * p.b_sb + (int64_t)pos0 * p.b_sr;
+    b_n = p.b_sr; b_k = p.b_sc;
+    klo = 0; khi = p.N;
+    m_hi = p.M - r0;
+    n_lo = p.lo - pos0; n_hi = p.hi - pos0;
+    ctiles = min(p.cspan, (TM + 2 * p.w - c0 + TN - 1) / TN);
+  } else if (PRIM == BAND_N) {
+    c0 = cg * TN;
+    const int pstart = r0 - p.w + p.off;                 // k <-> position pstart + k
+    a0 = p.a + ((int64_t)b * p.M + r0) * W;
+    a_m = W - 1; a_k = 1;
+    b0 = p.b + (int64_t)b * p.b_sb + (int64_t)pstart * p.b_sr + (int64_t)c0 * p.b_sc;
+    b_k = p.b_sr; b_n = p.b_sc;
+    m_hi = p.M - r0;
+    klo = max(p.lo - pstart, 0); khi = min(p.hi - pstart, min(m_hi, TM) + 2 * p.w);
+    n_hi = p.N - c0;
+  } else {
+    c0 = cg * TN;
+    const int istart = r0 - p.off - p.w;                 // k <-> band row istart + k, m <-> position r0 + m
+    a0 = p.a + ((int64_t)b * p.M + istart) * W + 2 * p.w;
+    a_m = 1; a_k = W - 1;
+    b0 = p.b + (int64_t)b * p.b_sb + (int64_t)istart * p.b_sr + (int64_t)c0 * p.b_sc;
+    b_k = p.b_sr; b_n = p.b_sc;
+    m_lo = p.lo - r0; m_hi = min(p.Mo, p.hi) - r0;       // positions outside the sequence (or the output) produce zeros
+    klo = max(-istart, max(m_lo, 0)); khi = min(p.M - istart, min(m_hi, TM) + 2 * p.w);
+    n_hi = p.N - c0;
+    if (m_hi <= 0) khi = klo;
+  }
+  const int kbeg = klo & ~(XK - 1);
+  const int kslices = khi > kbeg ? (khi - kbeg + XK - 1) / XK : 0;
+  const int nslices = kslices * ctiles;
+
+  // The next slice to load: reduction steps lk0 .. lk0 + 15 of column tile lct
+  int lsl = 0, lk0 = kbeg, lct = 0;
+  auto load_next = [&]() {
+    const int k0 = lk0;
+    float *As = smem + (lsl % STAGES) * STAGE, *Bs = As + A_FLOATS;
+    const int n0 = PRIM == BAND_NT ? lct * TN : 0;
+    // every element of the slice exists and, on band operands, lies in the band of every row of the tile
+    const bool inside = m_lo <= 0 && m_hi >= TM && n_lo <= n0 && n_hi >= n0 + TN && k0 >= klo && k0 + XK <= khi &&
+                        (PRIM == BAND_NT || (k0 >= TM - 1 && k0 + XK <= W));
+    // (one pointer per copy loop, advanced by a fixed step: no address arithmetic per element)
+    // ---- A ----
+    if (AKF) {
+      const int k = lane % XK, kk = k0 + k;
+      const float *src = a0 + (int64_t)(lane / XK) * a_m + (int64_t)kk * a_k;
+      const int64_t step = 2 * a_m;
+      const uint32_t dst = xsmem(As + k * AP + lane / XK);
+      if (inside) {
+#pragma unroll
+        for (int s = 0; s < TM / 2; s++, src += step) cp4(dst + s * 8, src, true);
+      } else {
+        const bool k_ok = kk >= klo && kk < khi;
+#pragma unroll 4
+        for (int s = 0; s < TM / 2; s++, src += step) {
+          const int m = lane / XK + 2 * s;
+          bool ok = k_ok && m < m_hi;
+          if (PRIM == BAND_N) ok = ok && kk >= m && kk < m + W;
+          cp4(dst + s * 8, ok ? src : p.a, ok);
+        }
+      }
+    } else {
+      constexpr int KS = XTHREADS / TM < 1 ? 1 : XTHREADS / TM;          // reduction steps per pass of the warp
+      constexpr int MS = TM / XTHREADS < 1 ? 1 : TM / XTHREADS;          // passes per reduction step
+#pragma unroll
+      for (int q = 0; q < MS; q++) {
+        const int m = q * XTHREADS + lane % TM, kfirst = k0 + lane / TM;
+        const float *src = a0 + m + (int64_t)kfirst * a_k;
+        const int64_t step = KS * a_k;
+        const uint32_t dst = xsmem(As + (lane / TM) * AP + m);
+        if (inside) {
+#pragma unroll
+          for (int s = 0; s < XK / KS; s++, src += step) cp4(dst + s * KS * AP * 4, src, true);
+        } else {
+          const int lo = m >= m_lo && m < m_hi ? max(klo, m) : khi, hi = min(khi, m + W);
+#pragma unroll 4
+          for (int s = 0; s < XK / KS; s++, src += step) {
+            const int kk = kfirst + s * KS;
+            const bool ok = kk >= lo && kk < hi;
+            cp4(dst + s * KS * AP * 4, ok ? src : p.a, ok);
+          }
+        }
+      }
+    }
+    // ---- B ----
+    if (!BKF && p.vec_b) {
+      constexpr int KS = XTHREADS * 4 / TN;
+      const int n = (lane % (TN / 4)) * 4, k = lane / (TN / 4);
+      const float *src = b0 + (int64_t)(k0 + k) * b_k + n;
+      const int64_t step = KS * b_k;
+      const uint32_t dst = xsmem(Bs + k * BP + n);
+#pragma unroll
+      for (int s = 0; s < XK / KS; s++, src += step) {
+        const int kk = k0 + k + s * KS;
+        const bool ok = inside || (n < n_hi && kk >= klo && kk < khi);
+        cp16(dst + s * KS * BP * 4, ok ? src : p.b, ok);
+      }
+    } else {
+      // BKF: lanes are 16 reduction steps x 2 columns; else 32 columns of one reduction step
+      const int n = BKF ? n0 + lane / XK : n0 + lane, k = BKF ? k0 + lane % XK : k0;
+#pragma unroll
+      for (int q = 0; q < (BKF ? 1 : TN / 32); q++) {
+        const float *src = b0 + (int64_t)k * b_k + (int64_t)(n + q * 32) * b_n;
+        const int64_t step = BKF ? 2 * b_n : b_k;
+        const uint32_t dst = xsmem(Bs + (k - k0) * BP + (n - n0) + q * 32);
+        constexpr int PASSES = BKF ? TN / 2 : XK;
+        if (inside) {
+#pragma unroll
+          for (int s = 0; s < PASSES; s++, src += step) cp4(dst + (BKF ? s * 8 : s * BP * 4), src, true);
+        } else {
+#pragma unroll 4
+          for (int s = 0; s < PASSES; s++, src += step) {
+            const int nn = BKF ? n + 2 * s : n + q * 32, kk = BKF ? k : k + s;
+            const bool ok = nn >= n_lo && nn < n_hi && kk >= klo && kk < khi;
+            cp4(dst + (BKF ? s * 8 : s * BP * 4), ok ? src : p.b, ok);
+          }
+        }
+      }
+    }
+    ++lsl;
+    lk0 += XK;
+    if (PRIM == BAND_NT && lk0 >= khi) {
+      lk0 = kbeg;
+      ++lct;
+    }
+  };
+
+  // acc[u][v][0] = {C(2u, 2v), C(2u+1, 2v+1)}, acc[u][v][1] = {C(2u, 2v+1), C(2u+1, 2v)}: the pairs of A are then used as
+  // they lie in shared memory and those of B once as they lie and once swapped, where {a, a} pairs would take a move per value.
+  uint64_t acc[MR / 2][MC / 2][2];
+  auto clear = [&]() {
+#pragma unroll
+    for (int u = 0; u < MR / 2; u++)
+#pragma unroll
+      for (int v = 0; v < MC / 2; v++) acc[u][v][0] = acc[u][v][1] = 0ull;
+  };
+  auto result = [&](int u, int v) -> float {
+    const float2 f = halves(acc[u / 2][v / 2][(u ^ v) & 1]);
+    return (u & 1) ? f.y : f.x;
+  };
+  // band_nt: the finished column tile goes out through shared memory (a staging buffer that is free), 32 columns at a
+  // time, so that the warp writes runs of 32 neighbouring band slots.
+  auto store_band = [&](int ctile, float *os) {
+#pragma unroll
+    for (int h = 0; h < MC / 4; h++) {
+      __syncwarp();
+#pragma unroll
+      for (int u = 0; u < MR; u++)
+        *reinterpret_cast<float4 *>(os + row_of(u) * OUT_P + tx * 4) =
+            make_float4(result(u, h * 4), result(u, h * 4 + 1), result(u, h * 4 + 2), result(u, h * 4 + 3));
+      __syncwarp();
+      const int n0 = ctile * TN + h * 32, n = n0 + lane;   // (in the coordinates of n_lo, n_hi)
+      float *dst = p.o + ((int64_t)b * p.M + r0) * W + (c0 + n);
+      const int64_t step = W - 1;
+      if (m_hi >= TM && n0 >= n_lo && n0 + 32 <= n_hi && c0 + n0 >= TM - 1 && c0 + n0 + 32 <= W) {   // all of it band, all in sequence
+#pragma unroll 8
+        for (int r = 0; r < TM; r++, dst += step) *dst = os[r * OUT_P + lane];
+      } else {
+        const bool in_seq = n >= n_lo && n < n_hi;
+        const int r_lo = max(c0 + n - W + 1, 0), r_hi = min(min(c0 + n + 1, TM), m_hi);   // rows that have this column in their band
+#pragma unroll 4
+        for (int r = 0; r < TM; r++, dst += step)
+          if (r >= r_lo && r < r_hi) *dst = in_seq ? os[r * OUT_P + lane] : 0.0f;
+      }
+    }
+    __syncwarp();
+  };
+
+  clear();
+#pragma unroll 1
+  for (int s = 0; s < STAGES - 1; s++) {
+    if (s < nslices) load_next();
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  int ck0 = kbeg, cct = 0;
+  for (int sl = 0; sl < nslices; sl++) {
+    if (sl + STAGES - 1 < nslices) load_next();          // (into the buffer of slice sl - 1, which the whole warp has left)
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
+    __syncwarp();                                        // slice sl has landed for every lane
+    float *As = smem + (sl % STAGES) * STAGE;
+    const float *Bs = As + A_FLOATS;
+#pragma unroll
+    for (int k = 0; k < XK; k++) {
+      uint64_t aa[MR / 2], bb[MC / 2], bs[MC / 2];
+      if (MR >= 4) {
+#pragma unroll
+        for (int u = 0; u < MR; u += 4) {
+          const ulonglong2 t = *reinterpret_cast<const ulonglong2 *>(As + k * AP + row_of(u));
+          aa[u / 2] = t.x;
+          aa[u / 2 + (MR >= 4 ? 1 : 0)] = t.y;
+        }
+      } else {
+        aa[0] = *reinterpret_cast<const uint64_t *>(As + k * AP + row_of(0));
+      }
+#pragma unroll
+      for (int v = 0; v < MC; v += 4) {
+        const float4 t = *reinterpret_cast<const float4 *>(Bs + k * BP + col_of(v));
+        bb[v / 2] = pair(t.x, t.y);
+        bb[v / 2 + 1] = pair(t.z, t.w);
+        bs[v / 2] = pair(t.y, t.x);
+        bs[v / 2 + 1] = pair(t.w, t.z);
+      }
+#pragma unroll
+      for (int u = 0; u < MR / 2; u++)
+#pragma unroll
+        for (int v = 0; v < MC / 2; v++) {
+          fma2(acc[u][v][0], aa[u], bb[v]);
+          fma2(acc[u][v][1], aa[u], bs[v]);
+        }
+    }
+    __syncwarp();
+    if (PRIM == BAND_NT) {
+      ck0 += XK;
+      if (ck0 >= khi) {
+        store_band(cct, As);
+        clear();
+        ck0 = kbeg;
+        ++cct;
+      }
+    }
+  }
+
+  if (PRIM == BAND_NT) {
+    if (kslices == 0)                                    // an empty reduction: every slot is zero
+      for (int t = 0; t < ctiles; t++) store_band(t, smem);
+  } else {
+    const int rmax = (PRIM == BAND_N ? p.M : p.Mo) - r0;
+    float *o0 = p.o + (int64_t)b * p.o_sb + (int64_t)r0 * p.o_sr + (int64_t)c0 * p.o_sc;
+#pragma unroll
+    for (int u = 0; u < MR; u++) {
+      const int m = row_of(u);
+      if (m >= rmax) continue;
+#pragma unroll
+      for (int v = 0; v < MC; v += 4) {
+        const int n = col_of(v);
+        float *dst = o0 + (int64_t)m * p.o_sr + (int64_t)n * p.o_sc;
+        if (p.vec_o) {
+          if (n < n_hi) *reinterpret_cast<float4 *>(dst) = make_float4(result(u, v), result(u, v + 1), result(u, v + 2), result(u, v + 3));
+        } else {
+          if (n < n_hi) dst[0] = result(u, v);
+          if (n + 1 < n_hi) dst[p.o_sc] = result(u, v + 1);
+          if (n + 2 < n_hi) dst[2 * p.o_sc] = result(u, v + 2);
+          if (n + 3 < n_hi) dst[3 * p.o_sc] = result(u, v + 3);
+        }
+      }
+    }
+  }
+}
+
+// 16-byte accesses along the hidden index: unit stride, whole groups of four, and every row starts on 16 bytes
+bool rows_of_16(const void *data, int64_t sb, int64_t sr, int64_t sc, int N) {
+  return ((uintptr_t)data & 15) == 0 && sc == 1 && (sr & 3) == 0 && (sb & 3) == 0 && (N & 3) == 0;
+}
+
+template <int PRIM, int MR, int MC> cudaError_t launch_tile(const Problem &p, cudaStream_t stream) {
+  constexpr int TM = 4 * MR, TN = 8 * MC;
+  const int rows = PRIM == BAND_T ? p.Mo : p.M;
+  ExactParams k;
+  k.a = static_cast<const float *>(p.a);
+  k.b = static_cast<const float *>(p.b);
+  k.o = static_cast<float *>(p.o);
+  k.a_sb = p.a_sb; k.a_sr = p.a_sr; k.a_sc = p.a_sc;
+  k.b_sb = p.b_sb; k.b_sr = p.b_sr; k.b_sc = p.b_sc;
+  k.o_sb = p.o_sb; k.o_sr = p.o_sr; k.o_sc = p.o_sc;
+  k.M = p.M; k.N = p.N; k.w = p.w; k.Mo = p.Mo; k.off = p.off; k.lo = p.lo; k.hi = p.hi;
+  k.nrt = (rows + TM - 1) / TM;
+  const int ctiles = PRIM == BAND_NT ? (int)(((int64_t)TM + 2 * (int64_t)p.w + TN - 1) / TN) : (p.N + TN - 1) / TN;
+  k.cspan = 1;
+  if (PRIM == BAND_NT) {   // all column tiles of a row tile in one warp once that gives every scheduler of the chip four warps
+    const int64_t rts = (int64_t)p.B * k.nrt;
+    const int64_t groups = (2368 + rts - 1) / rts;
+    k.cspan = groups >= ctiles ? 1 : (int)((ctiles + groups - 1) / groups);
+  }
+  k.nct = (ctiles + k.cspan - 1) / k.cspan;
+  k.vec_b = PRIM != BAND_NT && rows_of_16(p.b, p.b_sb, p.b_sr, p.b_sc, p.N);
+  k.vec_o = PRIM != BAND_NT && rows_of_16(p.o, p.o_sb, p.o_sr, p.o_sc, p.N);
+  const bool bkf = PRIM == BAND_NT ? p.b_sc <= p.b_sr : p.b_sr < p.b_sc;
+  const int64_t blocks = (int64_t)p.B * k.nrt * k.nct;
+  if (blocks <= 0) return cudaSuccess;
+  if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+  if (bkf)
+    band_exact32_kernel<PRIM, MR, MC, true><<<(unsigned)blocks, XTHREADS, 0, stream>>>(k);
+  else
+    band_exact32_kernel<PRIM, MR, MC, false><<<(unsigned)blocks, XTHREADS, 0, stream>>>(k);
+  return cudaGetLastError();
+}
+
+// The largest tile that still gives the chip's 592 warp schedulers enough warps: a tile costs reads in proportion to its
+// edges, but a scheduler with less than about two warps waits for its own loads and additions.  Measured (us):
+//   band_n  B=96 M=4096 N=64 w=256 (12288 tiles of 32 rows): 32 rows 568, 16 rows 640, 8 rows 996
+//           B=16 M=1024 N=64 w=64 (512): 13.2, 11.5, 16.5;   B=4 M=1024 N=64 w=64 (128): 12.2, 7.2, 6.8
+//   band_nt B=64 M=500 N=33 w=100 (4096 tiles of 32 x 64): 32x64 36.1, 32x32 39.1, 16x32 41.5
+//           M=2080 N=96 w=386 (845): 17.1, 15.1, 19.6;   B=4 M=1024 N=64 w=64 (384): 9.1, 8.1, 7.4;   M=400 w=8 (13): 9.1, 6.0, 4.5, 8x32 3.7
+template <int PRIM> cudaError_t launch_exact(const Problem &p, cudaStream_t stream) {
+  const int64_t rows = PRIM == BAND_T ? p.Mo : p.M;
+  if constexpr (PRIM == BAND_NT) {
+    const int64_t tiles = (int64_t)p.B * ((rows + 31) / 32) * ((32 + 2 * (int64_t)p.w + 63) / 64);
+    if (tiles >= 1184) return launch_tile<PRIM, 8, 8>(p, stream);
+    if (tiles >= 592) return launch_tile<PRIM, 8, 4>(p, stream);
+    if (tiles >= 148) return launch_tile<PRIM, 4, 4>(p, stream);
+    return launch_tile<PRIM, 2, 4>(p, stream);
+  } else {
+    const bool narrow = p.N <= 32;
+    const int64_t cols = (p.N + 63) / 64;
+    const int mr = p.B * ((rows + 31) / 32) * cols >= 1184 ? 8 : p.B * ((rows + 15) / 16) * cols >= 592 ? 4 : 2;
+    if (narrow) return mr == 8 ? launch_tile<PRIM, 8, 4>(p, stream) : mr == 4 ? launch_tile<PRIM, 4, 4>(p, stream) : launch_tile<PRIM, 2, 4>(p, stream);
+    return mr == 8 ? launch_tile<PRIM, 8, 8>(p, stream) : mr == 4 ? launch_tile<PRIM, 4, 8>(p, stream) : launch_tile<PRIM, 2, 8>(p, stream);
+  }
+}
+
+}  // namespace
+
+cudaError_t launch_exact32(Primitive prim, const Problem &p, cudaStream_t stream) {
+  switch (prim) {
+    case BAND_NT: return launch_exact<BAND_NT>(p, stream);
+    case BAND_N: return launch_exact<BAND_N>(p, stream);
+    default: return launch_exact<BAND_T>(p, stream);
+  }
+}
+
+}  // namespace wmm

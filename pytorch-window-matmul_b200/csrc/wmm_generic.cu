@@ -1,8 +1,8 @@
 // CUDA-core kernels for the three banded contractions: any dtype, any shape, any strides.
 //
-// This family is (a) the exact-ordering path for fp32 / fp64 -- every output element is one sequential
-// multiply-add chain over the ascending reduction index, one thread per output, no split-K and no
-// cross-thread partial sums, which is the accumulation order of the reference's kernels
+// This family is (a) the exact-ordering path for fp64 and, with split rounding, fp32 (fused fp32: wmm_exact32.cu) -- every
+// output element is one sequential multiply-add chain over the ascending reduction index, one thread per output, no
+// split-K and no cross-thread partial sums, which is the accumulation order of the reference's kernels
 // (csrc/window_matmul/cuda/window_matmul_cuda.cu:24-35,64-83) and of its CPU loops
 // (csrc/window_matmul/cpu/window_matmul_cpu.cpp:43,92-93,137,186-187) -- and (b) the path for shapes
 // the tensor-core kernels cannot take (hidden size 3, one-row sequences, odd windows, unaligned
@@ -281,7 +281,7 @@ cudaError_t launch_generic(Primitive prim, const Problem &p, cudaStream_t stream
     case WMM_F16: e = launch_prim<__half, false>(prim, p, stream); break;
     case WMM_BF16: e = launch_prim<__nv_bfloat16, false>(prim, p, stream); break;
     case WMM_F32:
-      e = split ? launch_prim<float, true>(prim, p, stream) : launch_prim<float, false>(prim, p, stream);
+      e = split ? launch_prim<float, true>(prim, p, stream) : launch_exact32(prim, p, stream);
       break;
     default:
       e = split ? launch_prim<double, true>(prim, p, stream) : launch_prim<double, false>(prim, p, stream);

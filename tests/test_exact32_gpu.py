@@ -1,0 +1,112 @@
+"""The fp32 kernels in exact order (csrc/wmm_exact32.cu): every tile size, at the edges of tiles, slices and sequences."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def wm():
+    import importlib
+
+    return importlib.import_module("window_matmul.window_matmul")
+
+
+def _dense(band, Mo, w, off, lo, hi):
+    """(B, M, 2w+1) -> the dense (B, M, Mo) float64 matrix with zeros outside the band and the sequence."""
+    B, M, W = band.shape
+    d = torch.zeros(B, M, Mo, dtype=torch.float64, device=band.device)
+    i = torch.arange(M, device=band.device)[:, None]
+    pos = i + torch.arange(W, device=band.device)[None, :] - w + off
+    ok = (pos >= lo) & (pos < hi)
+    ii = i.expand(M, W)[ok]
+    d[:, ii, pos[ok]] = band.double()[:, ok]
+    return d, ok
+
+
+def _check(got, want, absolute, terms, what):
+    """A chain of n fused multiply-adds is within n * 2^-24 * sum |a||b| of the exact sum (first order; 1 % on top)."""
+    bound = 1.01 * terms * 2.0 ** -24 * absolute
+    err = (got.double() - want).abs()
+    assert (err <= bound).all(), "%s: %.3g over the bound" % (what, float((err - bound).max()))
+
+
+# (batch, rows, hidden, window): the last ones take the 32-row tiles, the first ones the 8-row tiles
+SHAPES = [(1, 1, 1, 1), (2, 31, 3, 4), (1, 33, 64, 300), (2, 130, 65, 16), (3, 257, 20, 37), (40, 70, 33, 24), (30, 333, 48, 50), (70, 555, 64, 19), (41, 1030, 24, 70)]
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("position_major", [False, True])
+def test_exact32_against_float64(wm, shape, position_major):
+    B, M, N, w = shape
+    W = 2 * w + 1
+    g = torch.Generator(device="cuda")
+    g.manual_seed(3)
+    x = torch.randn(B, M, N, device="cuda", generator=g)
+    y = torch.randn(B, M, N, device="cuda", generator=g)
+    if position_major:
+        y = y.transpose(1, 2).contiguous().transpose(1, 2)
+    band = torch.randn(B, M, W, device="cuda", generator=g)
+    dense, ok = _dense(band, M, w, 0, 0, M)
+    band[:, ~ok] = float("nan")                      # out-of-sequence slots never reach a sum
+    out = wm.band_nt(x, y, w)
+    full = x.double() @ y.double().transpose(1, 2)
+    mag = x.double().abs() @ y.double().abs().transpose(1, 2)
+    i = torch.arange(M, device="cuda")[:, None].expand(M, W)[ok]
+    p = (torch.arange(M, device="cuda")[:, None] + torch.arange(W, device="cuda")[None, :] - w)[ok]
+    _check(out[:, ok], full[:, i, p], mag[:, i, p], N, "band_nt")
+    assert (out[:, ~ok] == 0).all()
+    _check(wm.band_n(band, y, w), dense @ y.double(), dense.abs() @ y.double().abs(), W, "band_n")
+    _check(wm.band_t(band, y, w), dense.transpose(1, 2) @ y.double(), dense.abs().transpose(1, 2) @ y.double().abs(), W, "band_t")
+
+
+@pytest.mark.parametrize("geometry", [(60, 140, 40, 0, 140), (200, 300, 50, 10, 280), (64, 64, -20, 5, 60)])
+def test_exact32_shard_geometry(wm, geometry):
+    """Rows of a shard against another row space: offset and in-sequence range as a sequence shard passes them."""
+    M, Mo, off, lo, hi = geometry
+    B, N, w = 2, 40, 30
+    W = 2 * w + 1
+    g = torch.Generator(device="cuda")
+    g.manual_seed(4)
+    x, y = torch.randn(B, M, N, device="cuda", generator=g), torch.randn(B, Mo, N, device="cuda", generator=g)
+    y[:, :lo] = float("nan")
+    y[:, hi:] = float("nan")
+    band = torch.randn(B, M, W, device="cuda", generator=g)
+    dense, ok = _dense(band, Mo, w, off, lo, hi)
+    band[:, ~ok] = float("nan")
+    yz = torch.nan_to_num(y).double()
+    kw = dict(other_off=off, seq=(lo, hi))
+    out = wm.band_nt(x, y, w, **kw)
+    i = torch.arange(M, device="cuda")[:, None].expand(M, W)[ok]
+    p = (torch.arange(M, device="cuda")[:, None] + torch.arange(W, device="cuda")[None, :] - w + off)[ok]
+    _check(out[:, ok], (x.double() @ yz.transpose(1, 2))[:, i, p], (x.double().abs() @ yz.abs().transpose(1, 2))[:, i, p], N, "band_nt")
+    assert (out[:, ~ok] == 0).all()
+    _check(wm.band_n(band, y, w, **kw), dense @ yz, dense.abs() @ yz.abs(), W, "band_n")
+    _check(wm.band_t(band, x, w, other_rows=Mo, **kw), dense.transpose(1, 2) @ x.double(), dense.abs().transpose(1, 2) @ x.double().abs(), W, "band_t")
+
+
+def test_exact32_order_of_summation(wm):
+    """One chain over the ascending reduction index: a product of floats is exact in float64, so the chain can be followed
+    there, rounding to float32 after every step (a double rounding may differ in a bit once in 2^29 steps)."""
+    B, M, N, w = 1, 90, 64, 40
+    W = 2 * w + 1
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    x, y = torch.randn(B, M, N, device="cuda", generator=g), torch.randn(B, M, N, device="cuda", generator=g)
+    band = torch.randn(B, M, W, device="cuda", generator=g)
+    dense, _ = _dense(band, M, w, 0, 0, M)
+    dense, xd, yd = dense[0].cpu().numpy(), x[0].double().cpu().numpy(), y[0].double().cpu().numpy()
+
+    def chain(a, b):   # (m, k), (k, n)
+        acc = np.zeros((a.shape[0], b.shape[1]), np.float32)
+        for k in range(a.shape[1]):
+            acc = (a[:, k:k + 1] * b[k:k + 1] + acc.astype(np.float64)).astype(np.float32)
+        return acc
+
+    assert np.mean(wm.band_n(band, y, w)[0].cpu().numpy() != chain(dense, yd)) < 1e-3
+    assert np.mean(wm.band_t(band, x, w)[0].cpu().numpy() != chain(dense.T.copy(), xd)) < 1e-3
+    want = chain(xd, yd.T.copy())
+    got, _ = _dense(wm.band_nt(x, y, w), M, w, 0, 0, M)
+    inside = np.abs(np.arange(M)[:, None] - np.arange(M)[None, :]) <= w
+    assert np.mean(got[0].cpu().numpy()[inside] != want[inside].astype(np.float64)) < 1e-3
