@@ -144,7 +144,8 @@ WMM_API int wmm_set_cta_limits(int contraction_ctas, int exchange_ctas);
  * waits runs out.  0 = clean.  Synchronises the current device.  Returns the word, or a negative status. */
 WMM_API int64_t wmm_device_status(int clear);
 /* Which kernel family the dispatcher picks for a problem: 0 = exact-order CUDA-core kernels, 1 = tcgen05
- * kernels, 2 = small-window kernels (w <= 32; warp-level MMAs fed from coalesced shared-memory tiles).  `primitive` is 1 (band_nt), 2 (band_n) or 3 (band_t); the operands carry the
+ * kernels fed by TMA, 2 = small-window kernels (w <= 32; warp-level MMAs fed from coalesced shared-memory tiles), 3 = tcgen05
+ * kernels fed by their own threads (16-bit, cols <= 128, sizes or addresses that TMA does not take).  `primitive` is 1 (band_nt), 2 (band_n) or 3 (band_t); the operands carry the
  * strides and alignment that decide; pass the same arguments as to the compute call.  Negative = status. */
 WMM_API int wmm_query_path(int primitive, const wmm_operand *a, const wmm_operand *b, const void *band,
                    const wmm_geometry *g, int dtype, unsigned flags);

@@ -109,11 +109,14 @@ void set_band_o(wmm::Problem &p, void *band) {
   p.o_sb = p.o_sr = p.o_sc = 0;
 }
 
-// Kernel family for a problem: 0 = exact-order CUDA-core kernels, 1 = tcgen05 kernels, 2 = small-window kernels.
+// Kernel family for a problem: 0 = exact-order CUDA-core kernels, 1 = tcgen05 kernels on TMA, 2 = small-window kernels,
+// 3 = tcgen05 kernels on loads by threads (16-bit problems that TMA cannot address).
 int pick_family(wmm::Primitive prim, const wmm::Problem &p) {
   if (p.flags & (WMM_FLAG_FORCE_GENERIC | WMM_FLAG_SPLIT_ROUNDING)) return 0;
   if (wmm::small_eligible(prim, p)) return 2;
   if (wmm::tensor_eligible(prim, p)) return 1;
+  // (WMM_FLAG_REQUIRE_TENSOR asks for families 1 and 2)
+  if (!(p.flags & WMM_FLAG_REQUIRE_TENSOR) && wmm::ragged_eligible(prim, p)) return 3;
   return 0;
 }
 
@@ -128,11 +131,12 @@ int dispatch(wmm::Primitive prim, const wmm::Problem &p, void *stream) {
   int launches = 0;
   cudaError_t e = family == 1   ? wmm::launch_tensor(prim, p, (cudaStream_t)stream, &launches)
                   : family == 2 ? wmm::launch_small(prim, p, (cudaStream_t)stream, &launches)
+                : family == 3 ? wmm::launch_ragged(prim, p, (cudaStream_t)stream, &launches)
                                 : wmm::launch_generic(prim, p, (cudaStream_t)stream, &launches);
   g_launches.fetch_add((uint64_t)launches, std::memory_order_relaxed);
   if (e != cudaSuccess)
     return fail(WMM_ERR_CUDA, "CUDA error launching primitive %d: %s [%s]", (int)prim, cudaGetErrorString(e),
-                family == 1 ? wmm::launch_detail() : family == 2 ? "small-window kernel launch" : "generic kernel launch");
+                family == 1 || family == 3 ? wmm::launch_detail() : family == 2 ? "small-window kernel launch" : "generic kernel launch");
   return WMM_OK;
 }
 

@@ -43,6 +43,9 @@ cudaError_t launch_exact32(Primitive prim, const Problem &p, cudaStream_t stream
 // alignment; `launch_tensor` must only be called when it holds.
 bool tensor_eligible(Primitive prim, const Problem &p);
 cudaError_t launch_tensor(Primitive prim, const Problem &p, cudaStream_t stream, int *launches);
+// The same for 16-bit problems that TMA cannot address (odd lengths, windows, hidden sizes, alignments; N <= 128).
+bool ragged_eligible(Primitive prim, const Problem &p);
+cudaError_t launch_ragged(Primitive prim, const Problem &p, cudaStream_t stream, int *launches);
 // band_n and band_t over the same band in ONE launch (the band is fetched from HBM once): `pn` and `pt`
 // are the two problems; eligibility includes that they share band, geometry and dtype.
 bool tensor_fused_pair_eligible(const Problem &pn, const Problem &pt);

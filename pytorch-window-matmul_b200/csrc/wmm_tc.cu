@@ -154,6 +154,7 @@ template <bool BF16> __device__ __forceinline__ uint16_t pack1(uint32_t bits) {
 #include "wmm_tc_mm.cuh"
 #include "wmm_tc_sweep.cuh"
 #include "wmm_tc_mm32.cuh"
+#include "wmm_tc_ragged.cuh"
 
 // ---------------------------------------------------------------------------------------------------
 // host side
@@ -472,6 +473,70 @@ template <bool BF16, int NH> cudaError_t launch_sweep(const Problem &pn, const P
   return launch_pdl(kern, grid, SWP_THREADS, S::ALLOC, stream, mband, my, mx, k);
 }
 
+// How rows of a (batch, rows, N) 16-bit tensor with unit column stride can be moved: in 16-byte pieces, words or elements.
+int row_mode(const void *data, int64_t sb, int64_t sr, int N, int B) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(data);
+  const int64_t s = sr | (B > 1 ? sb : 0) | N;
+  if ((a & 15) == 0 && (s & 7) == 0) return RAG_V16;
+  if ((a & 3) == 0 && (s & 1) == 0) return RAG_V4;
+  return RAG_V2;
+}
+// ... of an operand that may also be position-major (-1: neither index has unit stride)
+int operand_mode(const void *data, int64_t sb, int64_t sr, int64_t sc, int N, int B) {
+  if (sc == 1 || N == 1) return row_mode(data, sb, sr, N, B);
+  return sr == 1 ? RAG_POS : -1;
+}
+bool aligned4(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 3u) == 0; }
+
+void fill_ragged(RagParams &k, const Problem &p, int rows) {
+  k.a = static_cast<const uint16_t *>(p.a);
+  k.b = static_cast<const uint16_t *>(p.b);
+  k.o = static_cast<uint16_t *>(p.o);
+  k.a_sb = p.a_sb; k.a_sr = p.a_sr;
+  k.b_sb = p.b_sb; k.b_sr = p.b_sr; k.b_sc = p.b_sc;
+  k.o_sb = p.o_sb; k.o_sr = p.o_sr;
+  k.B = p.B; k.M = p.M; k.N = p.N; k.w = p.w; k.Mo = p.Mo; k.off = p.off; k.lo = p.lo; k.hi = p.hi;
+  k.tiles_per_batch = (rows + TILE - 1) / TILE;
+  k.total_tiles = k.tiles_per_batch * p.B;
+  k.parts = k.part_chunks = 1;
+  k.a_mode = row_mode(p.a, p.a_sb, p.a_sr, p.N, p.B);   // (band_nt)
+  k.b_mode = operand_mode(p.b, p.b_sb, p.b_sr, p.b_sc, p.N, p.B);
+  k.o_mode = row_mode(p.o, p.o_sb, p.o_sr, p.N, p.B);   // (band_n, band_t)
+}
+// Rows to tile: band_t may start its tiles one row early (an even band address), which can take one more tile.
+int ragged_rows(Primitive prim, const Problem &p) {
+  if (prim != BAND_T) return p.M;
+  return p.Mo + (((p.w - p.off) & 1) || ((p.M & 1) && p.B > 1) ? 1 : 0);
+}
+
+template <typename Kernel> cudaError_t launch_ragged_kernel(Kernel kern, const RagParams &k, int threads, int smem, cudaStream_t stream) {
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) {
+    set_launch_detail("cudaFuncSetAttribute(ragged kernel, %d bytes of shared memory)", smem);
+    return e;
+  }
+  const int64_t items = (int64_t)k.total_tiles * k.parts;
+  const int grid = persistent_grid(items < 0x7fffffffLL ? (int)items : 0x7fffffff);
+  set_launch_detail("ragged kernel launch, grid %d", grid);
+  return launch_pdl(kern, grid, threads, smem, stream, k);
+}
+template <bool BF16, int NH> cudaError_t launch_ragged_nh(Primitive prim, const Problem &p, cudaStream_t stream) {
+  RagParams k;
+  fill_ragged(k, p, ragged_rows(prim, p));
+  switch (prim) {
+    case BAND_NT: {
+      // fewer row tiles than SMs: a tile's chunks are spread over several CTAs (each reads the X tile again, from L2)
+      const int chunks = (int)(((int64_t)(p.M < TILE ? p.M : TILE) + 2ll * p.w + 1 + 63) / 64);
+      const int want = sm_count() / k.total_tiles;
+      k.part_chunks = want > 1 ? (chunks + want - 1) / want : chunks;
+      k.parts = (chunks + k.part_chunks - 1) / k.part_chunks;
+    }
+      return launch_ragged_kernel(band_nt_ragged_kernel<BF16, NH>, k, RNT_THREADS, RntSmem<NH>::ALLOC, stream);
+    case BAND_N: return launch_ragged_kernel(band_mm_ragged_kernel<BF16, NH, false>, k, RMM_THREADS, RmmSmem<NH>::ALLOC, stream);
+    default: return launch_ragged_kernel(band_mm_ragged_kernel<BF16, NH, true>, k, RMM_THREADS, RmmSmem<NH>::ALLOC, stream);
+  }
+}
+
 }  // namespace
 
 bool tensor_eligible(Primitive prim, const Problem &p) {
@@ -528,6 +593,27 @@ cudaError_t launch_tensor(Primitive prim, const Problem &p, cudaStream_t stream,
     e = launch_mm_any<0>(p, nullptr, stream);
   else if (prim == BAND_T)
     e = launch_mm_any<1>(p, nullptr, stream);
+  if (e == cudaSuccess && launches) ++*launches;
+  return e;
+}
+
+bool ragged_eligible(Primitive prim, const Problem &p) {
+  if (p.dtype != WMM_F16 && p.dtype != WMM_BF16) return false;
+  if (p.N < 1 || p.N > 128 || p.w < 1) return false;
+  if ((int64_t)p.B * (((int64_t)ragged_rows(prim, p) + TILE - 1) / TILE) > 0x7fffffffLL) return false;
+  if (operand_mode(p.b, p.b_sb, p.b_sr, p.b_sc, p.N, p.B) < 0) return false;
+  // The CUDA-core band_nt with one slice to reduce and at most one 64 x 64 tile per SM is over (2.4 us at 2 x 32 rows, N = 3)
+  // before these kernels have brought their first operands (9.8 us there; with N = 64, w = 50 and 500 rows 4.6 against 7.1).
+  if (prim == BAND_NT && p.N <= 16 && (int64_t)p.B * ((p.M + 63) / 64) * ((64 + 2 * (int64_t)p.w + 63) / 64) <= sm_count()) return false;
+  if (prim == BAND_NT) return aligned4(p.o) && (p.a_sc == 1 || p.N == 1);
+  return aligned4(p.a) && (p.o_sc == 1 || p.N == 1);
+}
+
+cudaError_t launch_ragged(Primitive prim, const Problem &p, cudaStream_t stream, int *launches) {
+  const bool bf16 = p.dtype == WMM_BF16;
+  cudaError_t e;
+  if (p.N <= 64) e = bf16 ? launch_ragged_nh<true, 64>(prim, p, stream) : launch_ragged_nh<false, 64>(prim, p, stream);
+  else e = bf16 ? launch_ragged_nh<true, 128>(prim, p, stream) : launch_ragged_nh<false, 128>(prim, p, stream);
   if (e == cudaSuccess && launches) ++*launches;
   return e;
 }

@@ -1,0 +1,623 @@
+// The three contractions on tensor cores for 16-bit problems that TMA cannot address: lengths, windows and hidden sizes
+// that fit no 16-byte pitch, operands at any even address.  Included by wmm_tc.cu (inside namespace wmm::<anon>).
+//
+// Tiles, accumulators and descriptors are those of the TMA kernels (128 rows, tcgen05.mma, fp32 sums in tensor memory); what
+// differs is how bytes get in and out.  Everything is moved in LINES: 64 consecutive elements = one 128-byte line of a swizzled
+// shared-memory tile.  A line is read by a warp, two elements per lane, checked against the range of elements that belong to
+// the band and the sequence (the others become zeros, so nothing else masks), and stored swizzled.
+//   * In the pitched view (wmm_tc.cu) a band row starts 2w elements after the one above it, an even number, so all lines of a
+//     tile start at the same parity.  Each tile picks its first column (band_nt), reduction index (band_n) or position
+//     (band_t) so that this parity is even: every band line is then read and written as aligned 4-byte words,
+//     whatever the window and the length are.
+//   * Operand rows take 16-byte pieces, 4-byte words or single elements, as their address and strides allow.
+//
+// band_n / band_t: reduction in chunks of 64.  Warps 0-3 epilogue, 4-19 loaders in two groups of eight that take chunks in turn
+// (one group's loads are in flight while the other stores), 20 MMA issuer.
+// band_nt: chunks of 64 positions.  Warps 0-15 epilogue (four groups of four, in turn), 16-23 loaders (four groups of two), 24 MMA issuer;
+// a finished 32 x 64 block goes through shared memory and out as one 128-byte line per row.
+//
+// What bounds them: the loads in flight per SM and the instructions that place them (46 % of the issue slots at 64 x 4001 rows,
+// N = 64, w = 255), at 0.4 to 0.5 of the memory rate; a line costs one load, one store and at its edges a mask kept as
+// one bit per line, where comparisons per line and element had cost a third of the time.  Measured (B200, us, CUDA cores before -> here):
+//                                        band_nt          band_n           band_t
+//   fp16 64 x 4001, N = 64, w = 255      763 -> 107       776 -> 110       808 -> 118      3.0 TB/s
+//   bf16 48 x 1111, N = 80, w = 75        90 ->  16       119 ->  17       123 ->  17      2.0 TB/s
+//   fp16 12 x 3001, N = 64, w = 128       62 ->  14        69 ->  13        79 ->  12
+//   fp16  1 x  500, N = 64, w = 50       7.1 -> 4.6      15.3 -> 5.7      16.3 -> 5.7
+
+constexpr unsigned long long ST_RAG_TIMEOUT = 1ull << 6;
+constexpr int RAG_STAGES = 4;
+constexpr int RMM_THREADS = 21 * 32, RNT_THREADS = 25 * 32;
+
+enum RagMode { RAG_V16 = 0, RAG_V4 = 1, RAG_V2 = 2, RAG_POS = 3 };   // operand rows in 16-byte, 4-byte or 2-byte pieces; position-major
+
+struct RagParams {
+  const uint16_t *a, *b;     // band_nt: X, Y; band_n / band_t: band, other operand
+  uint16_t *o;
+  int64_t a_sb, a_sr, b_sb, b_sr, b_sc, o_sb, o_sr;
+  int B, M, N, w, Mo, off, lo, hi;
+  int tiles_per_batch, total_tiles;
+  int parts, part_chunks;    // band_nt: a row tile's chunks are shared by `parts` work items of part_chunks each
+  int a_mode, b_mode, o_mode;
+};
+
+// word `lane` of line `row` in a tile of 128-byte lines with the 128-byte swizzle
+__device__ __forceinline__ uint32_t rag_word(uint32_t tile, int row, int lane) {
+  return tile + row * 128 + ((((lane >> 2) ^ row) & 7) << 4) + ((lane & 3) << 2);
+}
+__device__ __forceinline__ void sts32(uint32_t a, uint32_t v) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+__device__ __forceinline__ void sts128(uint32_t a, uint4 v) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t lds16(uint32_t a) {
+  uint16_t v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a) : "memory");
+  return v;
+}
+// bits u0 .. u1 - 1
+__device__ __forceinline__ uint32_t bit_range(int u0, int u1) {
+  const uint32_t below1 = u1 <= 0 ? 0u : u1 >= 32 ? 0xffffffffu : (1u << u1) - 1u;
+  const uint32_t below0 = u0 <= 0 ? 0u : u0 >= 32 ? 0xffffffffu : (1u << u0) - 1u;
+  return below1 & ~below0;
+}
+// elements 2 * lane and 2 * lane + 1 of the line at `line`, those outside [e0, e1) zero and not read
+__device__ __forceinline__ uint32_t line_pair(const uint16_t *line, int lane, int e0, int e1) {
+  const int e = 2 * lane;
+  uint32_t v = 0;
+  if (e >= e0 && e < e1) v = line[e];
+  if (e + 1 >= e0 && e + 1 < e1) v |= (uint32_t)line[e + 1] << 16;
+  return v;
+}
+
+// Loads ROWS rows (each one warp's share of a tile) of a (rows, N) operand with unit column stride into boxes of 128-byte lines:
+// row first + u exists for lo <= first + u < hi; the box of hidden columns 64x .. 64x+63 lies at tile + x * box_bytes.
+template <int ROWS, int NBOX>
+__device__ __forceinline__ void load_operand_rows(const uint16_t *base, int64_t sr, int N, int mode, int64_t first, int64_t lo, int64_t hi,
+                                                  uint32_t tile, uint32_t box_bytes, int line0, int lane) {
+  if (mode == RAG_V16) {
+    uint4 v[ROWS / 4][NBOX];
+#pragma unroll
+    for (int g = 0; g < ROWS / 4; g++) {
+      const int64_t r = first + g * 4 + (lane >> 3);
+#pragma unroll
+      for (int x = 0; x < NBOX; x++) {
+        const int h = x * 64 + (lane & 7) * 8;
+        v[g][x] = make_uint4(0, 0, 0, 0);
+        if (r >= lo && r < hi && h < N) v[g][x] = *reinterpret_cast<const uint4 *>(base + r * sr + h);
+      }
+    }
+#pragma unroll
+    for (int g = 0; g < ROWS / 4; g++) {
+      const int row = line0 + g * 4 + (lane >> 3);
+#pragma unroll
+      for (int x = 0; x < NBOX; x++) sts128(tile + x * box_bytes + row * 128 + ((((lane & 7) ^ row) & 7) << 4), v[g][x]);
+    }
+  } else {
+    constexpr int RB = ROWS < 16 / NBOX ? ROWS : 16 / NBOX;   // rows whose loads are in flight together
+#pragma unroll 1
+    for (int q = 0; q < ROWS; q += RB) {
+      uint32_t v[RB][NBOX];
+#pragma unroll
+      for (int u = 0; u < RB; u++) {
+        const int64_t r = first + q + u;
+#pragma unroll
+        for (int x = 0; x < NBOX; x++) {
+          v[u][x] = 0;
+          if (r >= lo && r < hi) {
+            const uint16_t *line = base + r * sr + x * 64;
+            if (mode == RAG_V4) {
+              if (x * 64 + 2 * lane < N) v[u][x] = *reinterpret_cast<const uint32_t *>(line + 2 * lane);
+            } else {
+              v[u][x] = line_pair(line, lane, 0, N - x * 64);
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < RB; u++)
+#pragma unroll
+        for (int x = 0; x < NBOX; x++) sts32(rag_word(tile + x * box_bytes, line0 + q + u, lane), v[u][x]);
+    }
+  }
+}
+// The same for a position-major operand (element (r, h) at base + h * sc + r): LINES lines, line h = 64 rows from `first` on.
+template <int LINES>
+__device__ __forceinline__ void load_position_lines(const uint16_t *base, int64_t sc, int N, int h0, int64_t first, int64_t lo, int64_t hi,
+                                                    uint32_t tile, int lane) {
+  const int e0 = (int)max((int64_t)0, min((int64_t)64, lo - first)), e1 = (int)max((int64_t)0, min((int64_t)64, hi - first));
+#pragma unroll 1
+  for (int q = 0; q < LINES; q += 8) {
+    uint32_t v[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) v[u] = h0 + q + u < N ? line_pair(base + (h0 + q + u) * sc + first, lane, e0, e1) : 0u;
+#pragma unroll
+    for (int u = 0; u < 8; u++) sts32(rag_word(tile, h0 + q + u, lane), v[u]);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------
+// band_n (TR = false) and band_t (TR = true)
+// ---------------------------------------------------------------------------------------------------
+
+// A tile: output rows r0 .. r0+127 (those in [m_lo, m_hi) can be non-zero), reduction indices [klo, khi) in chunks of 64 from kbeg on.
+// Band element (m, k) at a0 + m * 2w + k (band_n) or a0 + k * 2w + m (band_t), in the band for m <= k < m + 2w + 1; the other
+// operand's row of index k is row k + brow.
+struct RagTile {
+  int b, r0, m_lo, m_hi, klo, khi, kbeg, nch, brow;
+  int64_t a0;
+};
+template <bool TR> __device__ __forceinline__ RagTile rag_tile(const RagParams &p, int tile) {
+  RagTile t;
+  const int W = 2 * p.w + 1;
+  t.b = tile / p.tiles_per_batch;
+  t.r0 = (tile % p.tiles_per_batch) * TILE;
+  const int64_t row0 = (int64_t)t.b * p.M;
+  if (!TR) {
+    t.brow = t.r0 - p.w + p.off;
+    t.m_lo = 0;
+    t.m_hi = min(p.M - t.r0, TILE);
+    t.klo = max(p.lo - t.brow, 0);
+    t.khi = min(p.hi - t.brow, t.m_hi + 2 * p.w);
+    t.a0 = (row0 + t.r0) * W;
+    t.kbeg = t.klo - (int)((t.klo + t.a0) & 1);      // a0 + kbeg is even
+  } else {
+    t.r0 -= (int)((row0 + p.w - p.off) & 1);         // a0 (below) is even
+    t.brow = t.r0 - p.off - p.w;
+    t.m_lo = max(p.lo - t.r0, 0);
+    t.m_hi = min(min(p.Mo, p.hi) - t.r0, TILE);
+    t.klo = max(-t.brow, t.m_lo);
+    t.khi = min(p.M - t.brow, t.m_hi + 2 * p.w);
+    t.a0 = (row0 + t.brow) * W + 2 * p.w;
+    t.kbeg = t.klo;
+  }
+  t.nch = (t.m_hi > t.m_lo && t.khi > t.klo) ? (t.khi - t.kbeg + 63) / 64 : 0;
+  return t;
+}
+
+template <int NH> struct RmmSmem {
+  static constexpr int NBOX = NH / 64;
+  static constexpr int A_BYTES = 128 * 128, B_BYTES = 64 * 128 * NBOX, STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr int OUT_PITCH = NH * 2 + 16;      // bytes: 16-byte stores by 32 rows do not collide
+  static constexpr int OFF_OUT = RAG_STAGES * STAGE_BYTES;
+  static constexpr int OFF_BARS = OFF_OUT + 128 * OUT_PITCH;
+  static constexpr int OFF_MISC = OFF_BARS + (2 * RAG_STAGES + 4) * 8;
+  static constexpr int ALLOC = OFF_MISC + 32 + 1024;
+};
+
+template <bool BF16, int NH, bool TR>
+__global__ void __launch_bounds__(RMM_THREADS, 1) band_mm_ragged_kernel(const RagParams p) {
+  using S = RmmSmem<NH>;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t *base_ptr = smem_raw + (base - smem_u32(smem_raw));
+  const uint32_t bars = base + S::OFF_BARS;
+  auto bar_full = [&](int s) { return bars + 8u * s; };
+  auto bar_empty = [&](int s) { return bars + 8u * (RAG_STAGES + s); };
+  auto bar_acc_full = [&](int s) { return bars + 8u * (2 * RAG_STAGES + s); };
+  auto bar_acc_empty = [&](int s) { return bars + 8u * (2 * RAG_STAGES + 2 + s); };
+  volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(base_ptr + S::OFF_MISC);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(base_ptr + S::OFF_MISC + 4);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < RAG_STAGES; s++) { mbar_init(bar_full(s), 8); mbar_init(bar_empty(s), 1); }
+    for (int s = 0; s < 2; s++) { mbar_init(bar_acc_full(s), 1); mbar_init(bar_acc_empty(s), 4); }
+    *abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == 20) {
+    tmem_alloc(base + S::OFF_MISC, 2 * NH);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  griddep_launch_dependents();
+  griddep_wait();
+
+  const int W = 2 * p.w + 1;
+  if (warp >= 4 && warp < 20) {
+    // ---------------- loaders ----------------
+    const int group = (warp - 4) >> 3, wl = (warp - 4) & 7;
+    int it = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; ok && tile < p.total_tiles; tile += gridDim.x) {
+      const RagTile t = rag_tile<TR>(p, tile);
+      const uint16_t *other = p.b + (int64_t)t.b * p.b_sb;
+      for (int c = 0; c < t.nch; ++c, ++it) {
+        if ((it & 1) != group) continue;
+        const int s = it % RAG_STAGES;
+        if (!(ok = mbar_wait(bar_empty(s), ((it / RAG_STAGES) & 1) ^ 1, abort_flag))) break;
+        const uint32_t a_tile = base + s * S::STAGE_BYTES, b_tile = a_tile + S::A_BYTES;
+        const int k0 = t.kbeg + c * 64;
+        // every band line of the chunk belongs to the band and the sequence from its first to its last element
+        const bool full = t.m_lo <= 0 && t.m_hi >= TILE && k0 >= t.klo && k0 + 64 <= t.khi && k0 >= TILE - 1 && k0 + 64 <= W;
+        uint32_t v[16];
+        // band lines of this warp: band_n rows m = 16 wl + u; band_t reduction rows k = 16 (wl % 4) + u of box wl / 4
+        const int first = TR ? (wl & 3) * 16 : wl * 16;
+        const uint16_t *line0 = TR ? p.a + t.a0 + (int64_t)(k0 + first) * (2 * p.w) + (wl >> 2) * 64
+                                   : p.a + t.a0 + (int64_t)first * (2 * p.w) + k0;
+        if (full) {
+          const uint32_t *src = reinterpret_cast<const uint32_t *>(line0) + lane;
+#pragma unroll
+          for (int u = 0; u < 16; u++, src += p.w) v[u] = *src;
+        } else {
+          // Lane's element of parity h belongs to the band and the sequence in lines u of a range: a bit mask over the lines.
+          auto lines_of = [&](int h) -> uint32_t {
+            int u0, u1;
+            if (!TR) {
+              const int k = k0 + 2 * lane + h;                   // (m <= k < m + W)
+              u0 = max(k - W + 1, t.m_lo) - first;
+              u1 = k >= t.klo && k < t.khi ? min(k + 1, t.m_hi) - first : 0;
+            } else {
+              const int m = (wl >> 2) * 64 + 2 * lane + h;
+              u0 = max(m, t.klo) - k0 - first;
+              u1 = m >= t.m_lo && m < t.m_hi ? min(m + W, t.khi) - k0 - first : 0;
+            }
+            return bit_range(u0, u1);
+          };
+          const uint32_t lines_lo = lines_of(0), lines_hi = lines_of(1);
+          // a word that ends past the tensor may hold its last element: where that can be, single elements are read
+          if (t.b == p.B - 1 && (TR ? t.brow + k0 + 64 >= p.M : t.r0 + TILE >= p.M)) {
+            const uint16_t *src = line0 + 2 * lane;
+#pragma unroll
+            for (int u = 0; u < 16; u++, src += 2 * p.w) {
+              v[u] = 0;
+              if ((lines_lo >> u) & 1) v[u] = src[0];
+              if ((lines_hi >> u) & 1) v[u] |= (uint32_t)src[1] << 16;
+            }
+          } else {
+            const uint32_t lines_any = lines_lo | lines_hi;
+            const uint32_t *src = reinterpret_cast<const uint32_t *>(line0) + lane;
+#pragma unroll
+            for (int u = 0; u < 16; u++, src += p.w) {
+              v[u] = 0;
+              if ((lines_any >> u) & 1) v[u] = *src;
+            }
+#pragma unroll
+            for (int u = 0; u < 16; u++) {   // (after all the loads are on their way)
+              if (!((lines_lo >> u) & 1)) v[u] &= 0xffff0000u;
+              if (!((lines_hi >> u) & 1)) v[u] &= 0x0000ffffu;
+            }
+          }
+        }
+        if (p.b_mode == RAG_POS)
+          load_position_lines<NH / 8>(other, p.b_sc, p.N, wl * (NH / 8), (int64_t)t.brow + k0, (int64_t)t.brow + t.klo, (int64_t)t.brow + t.khi, b_tile, lane);
+        else
+          load_operand_rows<8, S::NBOX>(other, p.b_sr, p.N, p.b_mode, (int64_t)t.brow + k0 + wl * 8, (int64_t)t.brow + t.klo,
+                                        (int64_t)t.brow + t.khi, b_tile, 64 * 128, wl * 8, lane);
+        const uint32_t a_box = TR ? a_tile + (wl >> 2) * 8192 : a_tile;
+#pragma unroll
+        for (int u = 0; u < 16; u++) sts32(rag_word(a_box, first + u, lane), v[u]);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_full(s));
+      }
+    }
+  } else if (warp == 20) {
+    // ---------------- MMA issuer ----------------
+    if (lane == 0) {
+      const bool pos = p.b_mode == RAG_POS;
+      // A: K-major rows of 64 reduction indices (band_n), or MN-major: 64 reduction rows of 2 x 64 positions (band_t).
+      // B: MN-major reduction rows of NBOX x 64 hidden columns, or K-major hidden lines of 64 reduction indices.
+      constexpr uint64_t ADESC = TR ? smem_desc_base(8192, 1024, 2u) : smem_desc_base(16, 1024, 2u);
+      constexpr uint32_t A_STEP = TR ? 2048 : 32;
+      const uint64_t bdesc = pos ? smem_desc_base(16, 1024, 2u) : smem_desc_base(8192, 1024, 2u);
+      const uint32_t b_step = pos ? 32 : 2048;
+      const uint32_t idesc = pos ? instr_desc_f16(BF16, TR, false, TILE, NH) : instr_desc_f16(BF16, TR, true, TILE, NH);
+      int it = 0, tit = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; ok && tile < p.total_tiles; tile += gridDim.x) {
+        const int nch = rag_tile<TR>(p, tile).nch;
+        if (nch == 0) continue;
+        const int as = tit & 1;
+        if (!(ok = mbar_wait(bar_acc_empty(as), ((tit >> 1) & 1) ^ 1, abort_flag))) break;
+        tc_fence_after_sync();
+        for (int c = 0; c < nch; ++c, ++it) {
+          const int s = it % RAG_STAGES;
+          if (!(ok = mbar_wait(bar_full(s), (it / RAG_STAGES) & 1, abort_flag))) break;
+          tc_fence_after_sync();
+          const uint32_t a_addr = base + s * S::STAGE_BYTES, b_addr = a_addr + S::A_BYTES;
+#pragma unroll
+          for (int k = 0; k < 4; k++)
+            umma_f16(tmem_base + as * NH, smem_desc(ADESC, a_addr + k * A_STEP), smem_desc(bdesc, b_addr + k * b_step), idesc, (c > 0 || k > 0) ? 1u : 0u);
+          umma_commit(bar_empty(s));
+        }
+        if (ok) umma_commit(bar_acc_full(as));
+        ++tit;
+      }
+    }
+  } else {
+    // ---------------- epilogue: thread <-> output row ----------------
+    const uint32_t stage = base + S::OFF_OUT + warp * 32 * S::OUT_PITCH;
+    const int rows_out = TR ? p.Mo : p.M;
+    int tit = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; ok && tile < p.total_tiles; tile += gridDim.x) {
+      const RagTile t = rag_tile<TR>(p, tile);
+      const int as = tit & 1;
+      if (t.nch > 0) {
+        if (!(ok = mbar_wait(bar_acc_full(as), (tit >> 1) & 1, abort_flag))) break;
+        tc_fence_after_sync();
+      }
+      const int row = t.r0 + warp * 32 + lane;
+      uint16_t *out = p.o + (int64_t)t.b * p.o_sb;
+#pragma unroll
+      for (int g = 0; g < NH / 32; g++) {
+        uint32_t v[32];
+        if (t.nch > 0) {
+          tmem_ld_x32(tmem_base + as * NH + g * 32 + ((uint32_t)(warp * 32) << 16), v);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int q = 0; q < 32; q++) v[q] = 0;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          const uint4 piece = make_uint4(pack2<BF16>(v[q * 8 + 0], v[q * 8 + 1]), pack2<BF16>(v[q * 8 + 2], v[q * 8 + 3]),
+                                         pack2<BF16>(v[q * 8 + 4], v[q * 8 + 5]), pack2<BF16>(v[q * 8 + 6], v[q * 8 + 7]));
+          const int h = g * 32 + q * 8;
+          if (p.o_mode == RAG_V16) {
+            if (row >= 0 && row < rows_out && h < p.N) *reinterpret_cast<uint4 *>(out + row * p.o_sr + h) = piece;
+          } else {
+            sts128(stage + lane * S::OUT_PITCH + h * 2, piece);
+          }
+        }
+      }
+      if (t.nch > 0) {
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_acc_empty(as));
+        ++tit;
+      }
+      if (p.o_mode != RAG_V16) {
+        __syncwarp();
+        const int first = t.r0 + warp * 32;
+        const int u_lo = max(0, -first), u_hi = min(32, rows_out - first);
+        for (int u = u_lo; u < u_hi; u++) {
+          uint16_t *dst = out + (int64_t)(first + u) * p.o_sr;
+          if (p.o_mode == RAG_V4) {
+#pragma unroll
+            for (int h = 0; h < NH; h += 64)
+              if (h + 2 * lane < p.N) *reinterpret_cast<uint32_t *>(dst + h + 2 * lane) = lds32(stage + u * S::OUT_PITCH + h * 2 + lane * 4);
+          } else {
+#pragma unroll
+            for (int h = 0; h < NH; h += 32)
+              if (h + lane < p.N) dst[h + lane] = (uint16_t)lds16(stage + u * S::OUT_PITCH + (h + lane) * 2);
+          }
+        }
+        __syncwarp();
+      }
+    }
+  }
+
+  tc_fence_before_sync();
+  __syncthreads();
+  if (*abort_flag) {   // let the MMAs in flight end before tensor memory and shared memory go
+    if (threadIdx.x == 0) atomicOr(&g_device_status, ST_RAG_TIMEOUT);
+    const uint64_t t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
+    __syncthreads();
+  }
+  if (warp == 20) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_base, 2 * NH);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------
+// band_nt
+// ---------------------------------------------------------------------------------------------------
+
+constexpr int RNT_ACC = 4;   // accumulator stages of 64 columns
+
+template <int NH> struct RntSmem {
+  static constexpr int NBOX = NH / 64;
+  static constexpr int X_BYTES = 128 * 128 * NBOX, Y_BYTES = 64 * 128 * NBOX;
+  static constexpr int OFF_Y = 2 * X_BYTES;
+  static constexpr int OFF_OUT = OFF_Y + RAG_STAGES * Y_BYTES;
+  static constexpr int OUT_PITCH = 144;              // bytes of a 64-column row: 16-byte stores by 32 rows do not collide
+  static constexpr int OFF_BARS = OFF_OUT + 16 * 32 * OUT_PITCH;
+  static constexpr int OFF_MISC = OFF_BARS + (2 * RAG_STAGES + 4 + 2 * RNT_ACC) * 8;
+  static constexpr int ALLOC = OFF_MISC + 32 + 1024;
+};
+
+// Columns of a tile: column n stands for the element n positions after the tile's first one, whose address is
+// a0 = (b M + r0)(2w+1) - delta, delta = its parity; row m's band slots are the columns [m + delta, m + delta + 2w + 1).
+template <bool BF16, int NH>
+__global__ void __launch_bounds__(RNT_THREADS, 1) band_nt_ragged_kernel(const RagParams p) {
+  using S = RntSmem<NH>;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t *base_ptr = smem_raw + (base - smem_u32(smem_raw));
+  const uint32_t bars = base + S::OFF_BARS;
+  auto bar_full = [&](int s) { return bars + 8u * s; };
+  auto bar_empty = [&](int s) { return bars + 8u * (RAG_STAGES + s); };
+  auto bar_x_full = [&](int s) { return bars + 8u * (2 * RAG_STAGES + s); };
+  auto bar_x_empty = [&](int s) { return bars + 8u * (2 * RAG_STAGES + 2 + s); };
+  auto bar_acc_full = [&](int s) { return bars + 8u * (2 * RAG_STAGES + 4 + s); };
+  auto bar_acc_empty = [&](int s) { return bars + 8u * (2 * RAG_STAGES + 4 + RNT_ACC + s); };
+  volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(base_ptr + S::OFF_MISC);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(base_ptr + S::OFF_MISC + 4);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < RAG_STAGES; s++) { mbar_init(bar_full(s), 2); mbar_init(bar_empty(s), 1); }
+    for (int s = 0; s < 2; s++) { mbar_init(bar_x_full(s), 8); mbar_init(bar_x_empty(s), 1); }
+    for (int s = 0; s < RNT_ACC; s++) { mbar_init(bar_acc_full(s), 1); mbar_init(bar_acc_empty(s), 4); }
+    *abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == 24) {
+    tmem_alloc(base + S::OFF_MISC, RNT_ACC * 64);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  griddep_launch_dependents();
+  griddep_wait();
+
+  const int W = 2 * p.w + 1;
+  auto tile_at = [&](int item, int &b, int &r0, int &delta, int &c0, int &c1) {   // its chunks are c0 .. c1-1
+    const int tile = item / p.parts;
+    c0 = (item % p.parts) * p.part_chunks;
+    b = tile / p.tiles_per_batch;
+    r0 = (tile % p.tiles_per_batch) * TILE;
+    delta = (int)(((int64_t)b * p.M) & 1);             // (r0 is even)
+    c1 = min(c0 + p.part_chunks, (min(p.M - r0, TILE) + 2 * p.w + delta + 63) / 64);
+  };
+
+  if (warp >= 16 && warp < 24) {
+    // ---------------- loaders ----------------
+    const int group = (warp - 16) >> 1, wl = warp & 1;
+    int it = 0, tit = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; ok && tile < p.total_tiles * p.parts; tile += gridDim.x, ++tit) {
+      int b, r0, delta, c0, c1;
+      tile_at(tile, b, r0, delta, c0, c1);
+      const uint16_t *x = p.a + (int64_t)b * p.a_sb, *y = p.b + (int64_t)b * p.b_sb;
+      const int xs = tit & 1;
+      if (!(ok = mbar_wait(bar_x_empty(xs), ((tit >> 1) & 1) ^ 1, abort_flag))) break;
+      load_operand_rows<16, S::NBOX>(x, p.a_sr, p.N, p.a_mode, r0 + (warp - 16) * 16, 0, p.M, base + xs * S::X_BYTES, 128 * 128, (warp - 16) * 16, lane);
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_x_full(xs));
+      for (int c = c0; c < c1; ++c, ++it) {
+        if ((it & 3) != group) continue;
+        const int s = it % RAG_STAGES;
+        if (!(ok = mbar_wait(bar_empty(s), ((it / RAG_STAGES) & 1) ^ 1, abort_flag))) break;
+        const uint32_t y_tile = base + S::OFF_Y + s * S::Y_BYTES;
+        const int64_t pos0 = (int64_t)r0 - p.w + p.off - delta + c * 64;
+        if (p.b_mode == RAG_POS)
+          load_position_lines<NH / 2>(y, p.b_sc, p.N, wl * (NH / 2), pos0, p.lo, p.hi, y_tile, lane);
+        else
+#pragma unroll 1
+          for (int q = 0; q < 32; q += 32 / S::NBOX)
+            load_operand_rows<32 / S::NBOX, S::NBOX>(y, p.b_sr, p.N, p.b_mode, pos0 + wl * 32 + q, p.lo, p.hi, y_tile, 64 * 128, wl * 32 + q, lane);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_full(s));
+      }
+    }
+  } else if (warp == 24) {
+    // ---------------- MMA issuer ----------------
+    if (lane == 0) {
+      const bool pos = p.b_mode == RAG_POS;
+      constexpr uint64_t ADESC = smem_desc_base(16, 1024, 2u);
+      const uint64_t bdesc = pos ? smem_desc_base(8192, 1024, 2u) : smem_desc_base(16, 1024, 2u);
+      const uint32_t idesc = pos ? instr_desc_f16(BF16, false, true, TILE, 64) : instr_desc_f16(BF16, false, false, TILE, 64);
+      const int ksteps = (p.N + 15) / 16;
+      int it = 0, tit = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; ok && tile < p.total_tiles * p.parts; tile += gridDim.x, ++tit) {
+        int b, r0, delta, c0, c1;
+        tile_at(tile, b, r0, delta, c0, c1);
+        const int xs = tit & 1;
+        if (!(ok = mbar_wait(bar_x_full(xs), (tit >> 1) & 1, abort_flag))) break;
+        if (c0 >= c1) umma_commit(bar_x_empty(xs));    // (a short last tile may leave a part without chunks)
+        for (int c = c0; c < c1; ++c, ++it) {
+          const int s = it % RAG_STAGES, as = it % RNT_ACC;
+          if (!(ok = mbar_wait(bar_acc_empty(as), ((it / RNT_ACC) & 1) ^ 1, abort_flag))) break;
+          if (!(ok = mbar_wait(bar_full(s), (it / RAG_STAGES) & 1, abort_flag))) break;
+          tc_fence_after_sync();
+          const uint32_t a_addr = base + xs * S::X_BYTES, b_addr = base + S::OFF_Y + s * S::Y_BYTES;
+          for (int k = 0; k < ksteps; k++) {
+            const uint32_t b_off = pos ? (uint32_t)k * 2048u : (uint32_t)(k >> 2) * 8192u + (uint32_t)(k & 3) * 32u;
+            umma_f16(tmem_base + as * 64, smem_desc(ADESC, a_addr + (uint32_t)(k >> 2) * 16384u + (uint32_t)(k & 3) * 32u),
+                     smem_desc(bdesc, b_addr + b_off), idesc, k > 0 ? 1u : 0u);
+          }
+          umma_commit(bar_empty(s));
+          if (c == c1 - 1) umma_commit(bar_x_empty(xs));
+          umma_commit(bar_acc_full(as));               // (last: the epilogue waits for it, so no commit outlives the CTA)
+        }
+      }
+    }
+  } else {
+    // ---------------- epilogue: thread <-> band row, then warp <-> line ----------------
+    const int group = warp >> 2, quarter = warp & 3;
+    const uint32_t stage = base + S::OFF_OUT + warp * 32 * S::OUT_PITCH;
+    int it = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; ok && tile < p.total_tiles * p.parts; tile += gridDim.x) {
+      int b, r0, delta, c0, c1;
+      tile_at(tile, b, r0, delta, c0, c1);
+      const int m0 = quarter * 32;
+      uint16_t *line0 = p.o + ((int64_t)b * p.M + r0) * W - delta + (int64_t)m0 * (2 * p.w);
+      const int rows = min(32, p.M - r0 - m0);
+      for (int c = c0; c < c1; ++c, ++it) {
+        if ((it & 3) != group) continue;
+        const int as = it % RNT_ACC;
+        if (!(ok = mbar_wait(bar_acc_full(as), (it / RNT_ACC) & 1, abort_flag))) break;
+        tc_fence_after_sync();
+        const int n0 = c * 64;
+        const bool any = !(rows <= 0 || n0 + 63 < m0 + delta || n0 > m0 + 31 + delta + 2 * p.w);   // the block holds band slots
+        if (any) {
+          const int64_t pos0 = (int64_t)r0 - p.w + p.off - delta + n0;
+          const bool in_seq = pos0 >= p.lo && pos0 + 64 <= p.hi;
+          const int e0 = (int)max((int64_t)-1, min((int64_t)64, p.lo - pos0)), e1 = (int)max((int64_t)0, min((int64_t)64, p.hi - pos0));
+#pragma unroll
+          for (int g = 0; g < 2; g++) {
+            uint32_t v[32];
+            tmem_ld_x32(tmem_base + as * 64 + g * 32 + ((uint32_t)m0 << 16), v);
+            tmem_ld_wait();
+            if (!in_seq) {                             // exact zeros outside the sequence, whatever the operands hold
+#pragma unroll
+              for (int q = 0; q < 32; q++)
+                if (g * 32 + q < e0 || g * 32 + q >= e1) v[q] = 0u;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+              sts128(stage + lane * S::OUT_PITCH + g * 64 + q * 16,
+                     make_uint4(pack2<BF16>(v[q * 8], v[q * 8 + 1]), pack2<BF16>(v[q * 8 + 2], v[q * 8 + 3]),
+                                pack2<BF16>(v[q * 8 + 4], v[q * 8 + 5]), pack2<BF16>(v[q * 8 + 6], v[q * 8 + 7])));
+          }
+        }
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_acc_empty(as));
+        if (!any) continue;
+        uint16_t *line = line0 + n0;
+        const uint32_t src = stage + lane * 4;
+        if (rows == 32 && n0 >= m0 + 31 + delta && n0 + 64 <= m0 + delta + W) {   // every row has all 64 columns in its band
+          uint32_t *dst = reinterpret_cast<uint32_t *>(line) + lane;
+#pragma unroll 8
+          for (int u = 0; u < 32; u++, dst += p.w) *dst = lds32(src + u * S::OUT_PITCH);
+        } else {
+          // rows that have this lane's first (second) element in their band: slot n0 + 2 lane (+ 1) - row - delta in [0, W)
+          const int e = n0 + 2 * lane - m0 - delta;
+          const uint32_t rows_lo = bit_range(e - W + 1, min(e + 1, rows)), rows_hi = bit_range(e - W + 2, min(e + 2, rows));
+          uint16_t *dst = line + 2 * lane;
+#pragma unroll 8
+          for (int u = 0; u < 32; u++, dst += 2 * p.w) {
+            const uint32_t x = lds32(src + u * S::OUT_PITCH);
+            if ((rows_lo & rows_hi) >> u & 1) *reinterpret_cast<uint32_t *>(dst) = x;
+            if ((rows_lo & ~rows_hi) >> u & 1) dst[0] = (uint16_t)x;
+            if ((rows_hi & ~rows_lo) >> u & 1) dst[1] = (uint16_t)(x >> 16);
+          }
+        }
+        __syncwarp();
+      }
+    }
+  }
+
+  tc_fence_before_sync();
+  __syncthreads();
+  if (*abort_flag) {   // let the MMAs in flight end before tensor memory and shared memory go
+    if (threadIdx.x == 0) atomicOr(&g_device_status, ST_RAG_TIMEOUT);
+    const uint64_t t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
+    __syncthreads();
+  }
+  if (warp == 24) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_base, RNT_ACC * 64);
+  }
+}

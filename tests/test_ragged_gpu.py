@@ -1,0 +1,109 @@
+"""The tensor-core kernels for 16-bit problems that TMA cannot address (csrc/wmm_tc_ragged.cuh), against float64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def wm():
+    import importlib
+
+    from window_matmul import _native
+
+    yield importlib.import_module("window_matmul.window_matmul")
+    assert _native.device_status() == 0
+
+
+def _dense(band, Mo, w, off, lo, hi):
+    B, M, W = band.shape
+    d = torch.zeros(B, M, Mo, dtype=torch.float64, device=band.device)
+    pos = torch.arange(M, device=band.device)[:, None] + torch.arange(W, device=band.device)[None, :] - w + off
+    ok = (pos >= lo) & (pos < hi)
+    d[:, torch.arange(M, device=band.device)[:, None].expand(M, W)[ok], pos[ok]] = band.double()[:, ok]
+    return d, ok, pos
+
+
+def _check(got, want, absolute, terms, what):
+    """Sums in fp32: within twice terms * 2^-24 * sum |a||b| (the tensor cores may truncate); then one rounding to the 16-bit
+    type (fp16: half a step of the subnormals at least)."""
+    unit = 2.0 ** -8 if got.dtype == torch.bfloat16 else 2.0 ** -11
+    bound = 1.02 * (2 * terms * 2.0 ** -24 * absolute + unit * want.abs()) + 2.0 ** -25
+    err = (got.double() - want).abs()
+    assert (err <= bound).all(), "%s: %.3g over the bound" % (what, float((err - bound).max()))
+
+
+def _layout(t, how):
+    """The same values at another place: contiguous, position-major, at an odd element offset with odd strides, or as a view per head."""
+    B, M, N = t.shape
+    if how == "position":
+        return t.transpose(1, 2).contiguous().transpose(1, 2)
+    if how == "odd":
+        big = torch.zeros(B, M + 1, N + 3, dtype=t.dtype, device=t.device)
+        big[:, 1:, 1:N + 1] = t
+        return big[:, 1:, 1:N + 1]
+    if how == "head":
+        big = torch.zeros(B, M, 2 * N, dtype=t.dtype, device=t.device)
+        big[..., N:] = t
+        return big[..., N:]
+    return t
+
+
+# (batch, rows, hidden, window): lengths and windows at the edges of tiles and chunks; odd band rows in odd batch entries;
+# hidden sizes for 16-byte, 4-byte and 2-byte pieces and both accumulator widths
+SHAPES = [(1, 1, 1, 1), (2, 32, 3, 4), (3, 127, 80, 75), (2, 128, 64, 129), (3, 129, 66, 3), (2, 257, 128, 64), (1, 50, 32, 266),
+          (3, 301, 65, 31), (2, 640, 48, 200), (5, 193, 16, 97), (2, 1111, 96, 33), (200, 131, 40, 20)]
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("how", ["plain", "position", "odd", "head"])
+def test_ragged_against_float64(wm, shape, dtype, how):
+    from window_matmul import _native as Nt
+
+    B, M, N, w = shape
+    W = 2 * w + 1
+    g = torch.Generator(device="cuda")
+    g.manual_seed(7)
+    x = _layout(torch.randn(B, M, N, device="cuda", generator=g).to(dtype), "plain" if how == "position" else how)
+    y = _layout(torch.randn(B, M, N, device="cuda", generator=g).to(dtype), how)
+    band = torch.randn(B, M, W, device="cuda", generator=g).to(dtype)
+    dense, ok, pos = _dense(band, M, w, 0, 0, M)
+    band[:, ~ok] = float("nan")                      # out-of-sequence slots never reach a sum
+    out = torch.full((B, M, W), float("nan"), dtype=dtype, device="cuda")
+    if N not in (32, 64, 128) and (N > 16 or B * M > 4000):
+        assert Nt.lib.wmm_query_path(1, Nt.operand(x), Nt.operand(y), out.data_ptr(), Nt.geometry(B, M, N, w), Nt.dtype_code(x), 0) == 3
+    wm.band_nt(x, y, w, out=out)
+    i = torch.arange(M, device="cuda")[:, None].expand(M, W)[ok]
+    full, mag = x.double() @ y.double().transpose(1, 2), x.double().abs() @ y.double().abs().transpose(1, 2)
+    _check(out[:, ok], full[:, i, pos[ok]], mag[:, i, pos[ok]], N, "band_nt")
+    assert (out[:, ~ok] == 0).all()
+    for name, got, a in (("band_n", wm.band_n, dense), ("band_t", wm.band_t, dense.transpose(1, 2))):
+        o = _layout(torch.full((B, M, N), float("nan"), dtype=dtype, device="cuda"), "plain" if how == "position" else how)
+        got(band, y, w, out=o)
+        _check(o, a @ y.double(), a.abs() @ y.double().abs(), W, name)
+
+
+@pytest.mark.parametrize("geometry", [(60, 140, 40, 0, 140), (201, 300, 51, 11, 283), (64, 64, -21, 5, 60), (130, 131, 3, 40, 40), (33, 500, 100, 0, 500)])
+def test_ragged_shard_geometry(wm, geometry):
+    """Rows of a shard against another row space; what lies outside the sequence may hold anything."""
+    M, Mo, off, lo, hi = geometry
+    B, N, w = 3, 41, 30
+    W = 2 * w + 1
+    g = torch.Generator(device="cuda")
+    g.manual_seed(8)
+    x = torch.randn(B, M, N, device="cuda", generator=g).half()
+    y = torch.randn(B, Mo, N, device="cuda", generator=g).half()
+    band = torch.randn(B, M, W, device="cuda", generator=g).half()
+    dense, ok, pos = _dense(band, Mo, w, off, lo, hi)
+    y[:, :lo], y[:, hi:] = float("nan"), float("nan")
+    band[:, ~ok] = float("nan")
+    yz = torch.nan_to_num(y).double()
+    kw = dict(other_off=off, seq=(lo, hi))
+    out = wm.band_nt(x, y, w, **kw)
+    i = torch.arange(M, device="cuda")[:, None].expand(M, W)[ok]
+    _check(out[:, ok], (x.double() @ yz.transpose(1, 2))[:, i, pos[ok]], (x.double().abs() @ yz.abs().transpose(1, 2))[:, i, pos[ok]], N, "band_nt")
+    assert (out[:, ~ok] == 0).all()
+    _check(wm.band_n(band, y, w, **kw), dense @ yz, dense.abs() @ yz.abs(), W, "band_n")
+    dt = dense.transpose(1, 2)
+    _check(wm.band_t(band, x, w, other_rows=Mo, **kw), dt @ x.double(), dt.abs() @ x.double().abs(), W, "band_t")
