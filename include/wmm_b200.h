@@ -143,6 +143,23 @@ WMM_API int wmm_set_cta_limits(int contraction_ctas, int exchange_ctas);
 /* Reads (and, if `clear` is non-zero, resets) the status word that a kernel sets when one of its bounded
  * waits runs out.  0 = clean.  Synchronises the current device.  Returns the word, or a negative status. */
 WMM_API int64_t wmm_device_status(int clear);
+/* The five compute calls over operands whose batch dimensions do not merge into one stride (the (B, H, M, N) view of a
+ * (B, M, H*N) projection): `outer` calls of the function without the suffix, the i-th with every tensor moved on by i times
+ * its entry of `strides` (elements, in the order of the arguments), on `stream` one after another.  `g` describes one of
+ * them.  The first status that is not WMM_OK ends the call.  (The reference copies such operands together,
+ * window_matmul/window_matmul.py:36-37,72-73.) */
+WMM_API int wmm_band_nt_outer(const wmm_operand *x, const wmm_operand *y, void *band, int outer, const int64_t strides[3],
+                              const wmm_geometry *g, int dtype, unsigned flags, void *stream);
+WMM_API int wmm_band_n_outer(const void *band, const wmm_operand *y, const wmm_operand *out, int outer, const int64_t strides[3],
+                             const wmm_geometry *g, int dtype, unsigned flags, void *stream);
+WMM_API int wmm_band_t_outer(const void *band, const wmm_operand *x, const wmm_operand *out, int outer, const int64_t strides[3],
+                             const wmm_geometry *g, int dtype, unsigned flags, void *stream);
+WMM_API int wmm_window_bwd_outer(const wmm_operand *q, const wmm_operand *kt, const void *grad_band, const wmm_operand *grad_q,
+                                 const wmm_operand *grad_kt, int outer, const int64_t strides[5], const wmm_geometry *g, int dtype,
+                                 unsigned flags, void *stream);
+WMM_API int wmm_unwindow_bwd_outer(const void *band, const wmm_operand *v, const wmm_operand *grad_o, void *grad_band,
+                                   const wmm_operand *grad_v, int outer, const int64_t strides[5], const wmm_geometry *g, int dtype,
+                                   unsigned flags, void *stream);
 /* Which kernel family the dispatcher picks for a problem: 0 = exact-order CUDA-core kernels, 1 = tcgen05
  * kernels fed by TMA, 2 = small-window kernels (w <= 32; warp-level MMAs fed from coalesced shared-memory tiles), 3 = tcgen05
  * kernels fed by their own threads (16-bit, cols <= 128, sizes or addresses that TMA does not take).  `primitive` is 1 (band_nt), 2 (band_n) or 3 (band_t); the operands carry the

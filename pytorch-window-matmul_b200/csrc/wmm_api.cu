@@ -447,4 +447,84 @@ int wmm_unwindow_bwd(const void *band, const wmm_operand *v, const wmm_operand *
   return WMM_OK;
 }
 
+// ---- one call per outer index (see include/wmm_b200.h) ----
+static wmm_operand shifted_op(const wmm_operand *op, int64_t bytes) {
+  wmm_operand r = *op;
+  if (r.data) r.data = static_cast<const char *>(r.data) + bytes;
+  return r;
+}
+static const void *shifted_in(const void *band, int64_t bytes) { return band ? static_cast<const char *>(band) + bytes : nullptr; }
+static void *shifted_out(void *band, int64_t bytes) { return band ? static_cast<char *>(band) + bytes : nullptr; }
+
+static int outer_ok(int outer, const int64_t *strides) {
+  if (outer < 0) return fail(WMM_ERR_SHAPE, "Input mismatch: negative outer extent %d", outer);
+  if (!strides) return fail(WMM_ERR_NULL, "outer strides are NULL");
+  return WMM_OK;
+}
+
+int wmm_band_nt_outer(const wmm_operand *x, const wmm_operand *y, void *band, int outer, const int64_t strides[3],
+                      const wmm_geometry *g, int dtype, unsigned flags, void *stream) {
+  if (int s = outer_ok(outer, strides)) return s;
+  if (!x || !y) return fail(WMM_ERR_NULL, "an operand is NULL");
+  const int64_t e = (int64_t)elem_size(dtype);
+  for (int64_t i = 0; i < outer; ++i) {
+    const wmm_operand xi = shifted_op(x, i * strides[0] * e), yi = shifted_op(y, i * strides[1] * e);
+    if (int s = wmm_band_nt(&xi, &yi, shifted_out(band, i * strides[2] * e), g, dtype, flags, stream)) return s;
+  }
+  return WMM_OK;
+}
+
+int wmm_band_n_outer(const void *band, const wmm_operand *y, const wmm_operand *out, int outer, const int64_t strides[3],
+                     const wmm_geometry *g, int dtype, unsigned flags, void *stream) {
+  if (int s = outer_ok(outer, strides)) return s;
+  if (!y || !out) return fail(WMM_ERR_NULL, "an operand is NULL");
+  const int64_t e = (int64_t)elem_size(dtype);
+  for (int64_t i = 0; i < outer; ++i) {
+    const wmm_operand yi = shifted_op(y, i * strides[1] * e), oi = shifted_op(out, i * strides[2] * e);
+    if (int s = wmm_band_n(shifted_in(band, i * strides[0] * e), &yi, &oi, g, dtype, flags, stream)) return s;
+  }
+  return WMM_OK;
+}
+
+int wmm_band_t_outer(const void *band, const wmm_operand *x, const wmm_operand *out, int outer, const int64_t strides[3],
+                     const wmm_geometry *g, int dtype, unsigned flags, void *stream) {
+  if (int s = outer_ok(outer, strides)) return s;
+  if (!x || !out) return fail(WMM_ERR_NULL, "an operand is NULL");
+  const int64_t e = (int64_t)elem_size(dtype);
+  for (int64_t i = 0; i < outer; ++i) {
+    const wmm_operand xi = shifted_op(x, i * strides[1] * e), oi = shifted_op(out, i * strides[2] * e);
+    if (int s = wmm_band_t(shifted_in(band, i * strides[0] * e), &xi, &oi, g, dtype, flags, stream)) return s;
+  }
+  return WMM_OK;
+}
+
+int wmm_window_bwd_outer(const wmm_operand *q, const wmm_operand *kt, const void *grad_band, const wmm_operand *grad_q,
+                         const wmm_operand *grad_kt, int outer, const int64_t strides[5], const wmm_geometry *g, int dtype,
+                         unsigned flags, void *stream) {
+  if (int s = outer_ok(outer, strides)) return s;
+  if (!q || !kt || !grad_q || !grad_kt) return fail(WMM_ERR_NULL, "an operand is NULL");
+  const int64_t e = (int64_t)elem_size(dtype);
+  for (int64_t i = 0; i < outer; ++i) {
+    const wmm_operand qi = shifted_op(q, i * strides[0] * e), ki = shifted_op(kt, i * strides[1] * e);
+    const wmm_operand gqi = shifted_op(grad_q, i * strides[3] * e), gki = shifted_op(grad_kt, i * strides[4] * e);
+    if (int s = wmm_window_bwd(&qi, &ki, shifted_in(grad_band, i * strides[2] * e), &gqi, &gki, g, dtype, flags, stream)) return s;
+  }
+  return WMM_OK;
+}
+
+int wmm_unwindow_bwd_outer(const void *band, const wmm_operand *v, const wmm_operand *grad_o, void *grad_band,
+                           const wmm_operand *grad_v, int outer, const int64_t strides[5], const wmm_geometry *g, int dtype,
+                           unsigned flags, void *stream) {
+  if (int s = outer_ok(outer, strides)) return s;
+  if (!v || !grad_o || !grad_v) return fail(WMM_ERR_NULL, "an operand is NULL");
+  const int64_t e = (int64_t)elem_size(dtype);
+  for (int64_t i = 0; i < outer; ++i) {
+    const wmm_operand vi = shifted_op(v, i * strides[1] * e), goi = shifted_op(grad_o, i * strides[2] * e);
+    const wmm_operand gvi = shifted_op(grad_v, i * strides[4] * e);
+    if (int s = wmm_unwindow_bwd(shifted_in(band, i * strides[0] * e), &vi, &goi, shifted_out(grad_band, i * strides[3] * e), &gvi, g, dtype, flags, stream))
+      return s;
+  }
+  return WMM_OK;
+}
+
 }  // extern "C"

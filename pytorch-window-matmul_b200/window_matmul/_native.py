@@ -96,6 +96,17 @@ def _load():
     lib.wmm_window_bwd.argtypes = [P(Operand), P(Operand), vp, P(Operand), P(Operand), P(Geometry), i32, u32, vp]
     lib.wmm_unwindow_bwd.restype = i32
     lib.wmm_unwindow_bwd.argtypes = [vp, P(Operand), P(Operand), vp, P(Operand), P(Geometry), i32, u32, vp]
+    i64p = P(ctypes.c_int64)
+    lib.wmm_band_nt_outer.restype = i32
+    lib.wmm_band_nt_outer.argtypes = [P(Operand), P(Operand), vp, i32, i64p, P(Geometry), i32, u32, vp]
+    lib.wmm_band_n_outer.restype = i32
+    lib.wmm_band_n_outer.argtypes = [vp, P(Operand), P(Operand), i32, i64p, P(Geometry), i32, u32, vp]
+    lib.wmm_band_t_outer.restype = i32
+    lib.wmm_band_t_outer.argtypes = [vp, P(Operand), P(Operand), i32, i64p, P(Geometry), i32, u32, vp]
+    lib.wmm_window_bwd_outer.restype = i32
+    lib.wmm_window_bwd_outer.argtypes = [P(Operand), P(Operand), vp, P(Operand), P(Operand), i32, i64p, P(Geometry), i32, u32, vp]
+    lib.wmm_unwindow_bwd_outer.restype = i32
+    lib.wmm_unwindow_bwd_outer.argtypes = [vp, P(Operand), P(Operand), vp, P(Operand), i32, i64p, P(Geometry), i32, u32, vp]
     lib.wmm_halo_pull.restype = i32
     lib.wmm_halo_pull.argtypes = [P(HaloBuffer), i32, P(HaloFlags), i32, i32, i32, i32, i32, i32, vp]
     lib.wmm_halo_pull_static.restype = i32
@@ -139,6 +150,22 @@ def geometry(batch, rows, cols, window, other_rows=None, other_off=0, seq=None, 
 
 def stream_of(t: torch.Tensor) -> ctypes.c_void_p:
     return ctypes.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
+
+
+# The current stream's handle without a Stream object around it (a tenth of the time), where torch has it.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda index: torch.cuda.current_stream(index).cuda_stream)
+
+
+def run(call, t: torch.Tensor, *args) -> None:
+    """call(*args, stream) on `t`'s device and its current stream; raises on a status that is not WMM_OK."""
+    index = t.get_device()
+    if index == torch.cuda.current_device():
+        status = call(*args, _raw_stream(index))
+    else:
+        with torch.cuda.device(index):
+            status = call(*args, _raw_stream(index))
+    if status != 0:
+        check(status)
 
 
 def check(status: int) -> None:

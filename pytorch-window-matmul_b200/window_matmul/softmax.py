@@ -42,9 +42,8 @@ def band_softmax(scores, scale=1.0, mask=True, *, other_off=0, seq=None, other_r
     w = (W - 1) // 2
     probs = torch.empty_like(scores) if out is None else _check_out(out, scores)
     g = N.geometry(B, M, 0, w, M if other_rows is None else other_rows, other_off, seq)
-    with torch.cuda.device(scores.device):
-        N.check(N.lib.wmm_band_softmax(scores.data_ptr(), probs.data_ptr(), g, N.dtype_code(scores), float(scale),
-                                       0 if mask else N.FLAG_SOFTMAX_KEEP_PADDING, N.stream_of(scores)))
+    N.run(N.lib.wmm_band_softmax, scores, scores.data_ptr(), probs.data_ptr(), g, N.dtype_code(scores), float(scale),
+          0 if mask else N.FLAG_SOFTMAX_KEEP_PADDING)
     return probs
 
 
@@ -59,19 +58,22 @@ def band_softmax_backward(probs, grad_probs, scale=1.0, mask=True, *, other_off=
     w = (W - 1) // 2
     grad_scores = torch.empty_like(probs) if out is None else _check_out(out, probs)
     g = N.geometry(B, M, 0, w, M if other_rows is None else other_rows, other_off, seq)
-    with torch.cuda.device(probs.device):
-        N.check(N.lib.wmm_band_softmax_bwd(probs.data_ptr(), grad_probs.data_ptr(), grad_scores.data_ptr(), g,
-                                           N.dtype_code(probs), float(scale),
-                                           0 if mask else N.FLAG_SOFTMAX_KEEP_PADDING, N.stream_of(probs)))
+    N.run(N.lib.wmm_band_softmax_bwd, probs, probs.data_ptr(), grad_probs.data_ptr(), grad_scores.data_ptr(), g,
+          N.dtype_code(probs), float(scale), 0 if mask else N.FLAG_SOFTMAX_KEEP_PADDING)
     return grad_scores
 
 
+def _flat(t: torch.Tensor) -> torch.Tensor:
+    return t if t.dim() == 3 else t.reshape(-1, t.shape[-2], t.shape[-1])
+
+
 class WindowSoftmaxFunc(torch.autograd.Function):
-    """Saves only the probabilities (the scores are not needed for the backward)."""
+    """Saves only the probabilities (the scores are not needed for the backward).  Leading dimensions are flattened inside:
+    as views outside they would be one more autograd node each."""
 
     @staticmethod
     def forward(ctx, scores: torch.Tensor, scale: float, mask: bool) -> torch.Tensor:
-        probs = band_softmax(scores, scale, mask)
+        probs = band_softmax(_flat(scores), scale, mask).view(scores.shape)
         ctx.save_for_backward(probs)
         ctx.scale, ctx.mask = scale, mask
         return probs
@@ -79,7 +81,7 @@ class WindowSoftmaxFunc(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_probs: torch.Tensor) -> Tuple[Optional[torch.Tensor], None, None]:
         (probs,) = ctx.saved_tensors
-        return band_softmax_backward(probs, grad_probs, ctx.scale, ctx.mask), None, None
+        return band_softmax_backward(_flat(probs), _flat(grad_probs), ctx.scale, ctx.mask).view(probs.shape), None, None
 
 
 def window_softmax(scores: torch.Tensor, scale: float = 1.0, mask: bool = True) -> torch.Tensor:
@@ -88,6 +90,4 @@ def window_softmax(scores: torch.Tensor, scale: float = 1.0, mask: bool = True) 
     _check(scores)
     if scores.numel() == 0:
         return scores.clone()
-    lead = scores.shape[:-2]
-    flat = scores.reshape(-1, scores.shape[-2], scores.shape[-1])
-    return WindowSoftmaxFunc.apply(flat, float(scale), bool(mask)).reshape(*lead, *scores.shape[-2:])
+    return WindowSoftmaxFunc.apply(scores, float(scale), bool(mask))

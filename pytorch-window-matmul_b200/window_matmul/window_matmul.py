@@ -29,6 +29,9 @@ def set_flags(flags: int) -> int:
 
 
 def _require_cuda(*tensors: torch.Tensor) -> None:
+    first = tensors[0]
+    if first.is_cuda and all(t.device == first.device and t.dtype == first.dtype for t in tensors[1:]):
+        return
     for t in tensors:
         if not t.is_cuda:
             raise RuntimeError("window_matmul: tensor must be CUDA tensor (this package has no CPU path)")
@@ -93,9 +96,7 @@ def band_nt(x, y, window, *, other_off=0, seq=None, out=None, flags=None):
     shape = (B, M, 2 * window + 1)
     band = torch.empty(shape, dtype=x.dtype, device=x.device) if out is None else _check_out(out, shape, x, True)
     g = N.geometry(B, M, Nn, window, y.shape[1], other_off, seq, _band_stride(band))
-    with torch.cuda.device(x.device):
-        N.check(N.lib.wmm_band_nt(N.operand(x), N.operand(y), band.data_ptr(), g, N.dtype_code(x),
-                                  _FLAGS if flags is None else flags, N.stream_of(x)))
+    N.run(N.lib.wmm_band_nt, x, N.operand(x), N.operand(y), band.data_ptr(), g, N.dtype_code(x), _FLAGS if flags is None else flags)
     return band
 
 
@@ -108,9 +109,7 @@ def band_n(band, y, window, *, rows_out=None, other_off=0, seq=None, out=None, f
     Nn = y.shape[2]
     o = torch.empty((B, M, Nn), dtype=y.dtype, device=y.device) if out is None else _check_out(out, (B, M, Nn), y, False)
     g = N.geometry(B, M, Nn, window, y.shape[1], other_off, seq, band_sb)
-    with torch.cuda.device(y.device):
-        N.check(N.lib.wmm_band_n(band.data_ptr(), N.operand(y), N.operand(o), g, N.dtype_code(y),
-                                 _FLAGS if flags is None else flags, N.stream_of(y)))
+    N.run(N.lib.wmm_band_n, y, band.data_ptr(), N.operand(y), N.operand(o), g, N.dtype_code(y), _FLAGS if flags is None else flags)
     return o
 
 
@@ -130,13 +129,12 @@ def band_t(band, x, window, *, other_rows=None, other_off=0, seq=None, out=None,
         _mismatch(edges.dim() == 3 and edges.shape[0] == B and edges.shape[2] == Nn and edges.shape[1] % 2 == 0
                   and 0 < edges.shape[1] <= Mo and edges.dtype == torch.float32 and edges.device == x.device
                   and edges.is_contiguous() and edges.data_ptr() % 16 == 0)
-    with torch.cuda.device(x.device):
-        if edges is not None:
-            N.check(N.lib.wmm_band_t_edges(band.data_ptr(), N.operand(x), N.operand(o), edges.data_ptr(), edges.shape[1] // 2, int(edge_skip), g,
-                                           N.dtype_code(x), _FLAGS if flags is None else flags, N.stream_of(x)))
-        else:
-            N.check(N.lib.wmm_band_t(band.data_ptr(), N.operand(x), N.operand(o), g, N.dtype_code(x),
-                                     _FLAGS if flags is None else flags, N.stream_of(x)))
+    flags = _FLAGS if flags is None else flags
+    if edges is not None:
+        N.run(N.lib.wmm_band_t_edges, x, band.data_ptr(), N.operand(x), N.operand(o), edges.data_ptr(), edges.shape[1] // 2, int(edge_skip), g,
+              N.dtype_code(x), flags)
+    else:
+        N.run(N.lib.wmm_band_t, x, band.data_ptr(), N.operand(x), N.operand(o), g, N.dtype_code(x), flags)
     return o
 
 
@@ -168,9 +166,8 @@ def window_matmul_backward(src, other, window_size, grad_output, need=(True, Tru
         gq = torch.empty((B, M, Nn), dtype=src.dtype, device=src.device) if out is None else _check_out(out[0], (B, M, Nn), src, False)
         gkt = torch.empty((B, M, Nn), dtype=src.dtype, device=src.device) if out is None else _check_out(out[1], (B, M, Nn), src, False)
         g = N.geometry(B, M, Nn, window_size)
-        with torch.cuda.device(src.device):
-            N.check(N.lib.wmm_window_bwd(N.operand(src), N.operand(kt), grad_output.data_ptr(), N.operand(gq),
-                                         N.operand(gkt), g, N.dtype_code(src), _FLAGS, N.stream_of(src)))
+        N.run(N.lib.wmm_window_bwd, src, N.operand(src), N.operand(kt), grad_output.data_ptr(), N.operand(gq), N.operand(gkt), g,
+              N.dtype_code(src), _FLAGS)
         return gq, gkt.transpose(-1, -2)
     gq = band_n(grad_output, kt, window_size) if need[0] else None
     gk = band_t(grad_output, src, window_size).transpose(-1, -2) if need[1] else None
@@ -201,9 +198,8 @@ def unwindow_matmul_backward(src, other, window_size, grad_output, need=(True, T
             else _check_out(out[0], (B, M, 2 * window_size + 1), src, True)
         gv = torch.empty((B, M, Nn), dtype=src.dtype, device=src.device) if out is None else _check_out(out[1], (B, M, Nn), src, False)
         g = N.geometry(B, M, Nn, window_size)
-        with torch.cuda.device(src.device):
-            N.check(N.lib.wmm_unwindow_bwd(src.data_ptr(), N.operand(other), N.operand(grad_output), ga.data_ptr(),
-                                           N.operand(gv), g, N.dtype_code(src), _FLAGS, N.stream_of(src)))
+        N.run(N.lib.wmm_unwindow_bwd, src, src.data_ptr(), N.operand(other), N.operand(grad_output), ga.data_ptr(), N.operand(gv), g,
+              N.dtype_code(src), _FLAGS)
         return ga, gv
     ga = band_nt(grad_output, other, window_size) if need[0] else None
     gv = band_t(src, grad_output, window_size) if need[1] else None
@@ -225,6 +221,8 @@ def _lead(t: torch.Tensor) -> int:
 
 
 def _viewable3(t: torch.Tensor) -> bool:
+    if t.dim() == 3 or t.is_contiguous():
+        return True
     try:
         t.view(_lead(t), t.shape[-2], t.shape[-1])   # (an explicit size: -1 is ambiguous for empty tensors)
         return True
@@ -249,41 +247,79 @@ def _slices(depth: int, shape) -> list:
 
 def _v3(t: torch.Tensor, idx) -> torch.Tensor:
     s = t[idx] if idx else t
-    return s.view(_lead(s), s.shape[-2], s.shape[-1])
+    return s if s.dim() == 3 else s.view(_lead(s), s.shape[-2], s.shape[-1])
+
+
+def _autocast(*tensors: torch.Tensor):
+    """What torch.amp.custom_fwd(device_type="cuda", cast_inputs=torch.float16) does to a forward's tensors (:9, :45): under
+    autocast they run in float16.  (The decorator itself enters an autocast context on every call; the kernels do not look.)"""
+    if not torch.is_autocast_enabled("cuda"):
+        return tensors
+    return tuple(t.to(torch.float16) if t.is_cuda and t.is_floating_point() and t.dtype != torch.float64 else t for t in tensors)
+
+
+def _grad_like(t: torch.Tensor) -> torch.Tensor:
+    """An uninitialised gradient of a strided operand, laid out as the operand where the kernels can write that densely: the
+    gradient of a per-head view then is a view of the projection's gradient and is not copied together."""
+    if t.stride(-1) == 1 and all(st > 0 for st in t.stride()):
+        g = torch.empty_like(t)
+        if g.stride(-1) == 1 and g.stride(-2) % 8 == 0:
+            return g
+    return torch.empty(t.shape, dtype=t.dtype, device=t.device)
+
+
+def _outer_call(call, depth: int, tensors, pack, geometry, code) -> None:
+    """call(...) for every outer index of the first `depth` dimensions, the innermost of them walked by the library.
+    `tensors` in the order of the call's arguments; pack[i] makes the argument of tensors[i]."""
+    lead = tensors[0].shape[:depth]
+    strides = (N.ctypes.c_int64 * len(tensors))(*[t.stride(depth - 1) for t in tensors])
+    for idx in _slices(depth - 1, lead):
+        first = [_v3(t[idx + (0,)], ()) for t in tensors]
+        N.run(call, first[0], *[p(t) for p, t in zip(pack, first)], lead[-1], strides, geometry, code, _FLAGS)
+
+
+def _outer_addressable(t: torch.Tensor, depth: int) -> torch.Tensor:
+    """An operand whose slices below `depth` are (batch, rows, cols) views the kernels can address well."""
+    return t if (t.stride(-1) == 1 or t.stride(-2) == 1) and _viewable3(t[(0,) * depth]) else t.contiguous()
 
 
 class _StridedWindowMatmulFunc(torch.autograd.Function):
-    """WindowMatmulFunc for operands whose leading dimensions do not merge: same kernels, one call per outer index."""
+    """WindowMatmulFunc for operands whose leading dimensions do not merge: same kernels, one launch per outer index."""
 
     @staticmethod
-    @torch.amp.custom_fwd(device_type="cuda", cast_inputs=torch.float16)
     def forward(ctx, inp, other, window_size, depth):
+        inp, other = _autocast(inp, other)
         _require_cuda(inp, other)
         *dims, M, Nh = inp.shape
         out = torch.empty((*dims, M, 2 * window_size + 1), dtype=inp.dtype, device=inp.device)
-        for idx in _slices(depth, inp.shape):
-            window_matmul_forward(_v3(inp, idx), _v3(other, idx), window_size, out=_v3(out, idx))
+        if out.numel():
+            x, y = _outer_addressable(inp, depth), _outer_addressable(other.transpose(-1, -2), depth)
+            g = N.geometry(_lead(inp[(0,) * depth]), M, Nh, window_size)
+            _outer_call(N.lib.wmm_band_nt_outer, depth, (x, y, out), (N.operand, N.operand, _pointer), g, N.dtype_code(inp))
         ctx.save_for_backward(inp, other)
         ctx.depth = depth
         return out
 
     @staticmethod
-    @torch.amp.custom_bwd(device_type="cuda")
     def backward(ctx, grad_output):
         inp, other = ctx.saved_tensors
-        window_size = grad_output.shape[-1] // 2
+        depth, window_size = ctx.depth, grad_output.shape[-1] // 2
+        _require_cuda(inp, other, grad_output)
         grad_output = grad_output.contiguous()
-        need = tuple(ctx.needs_input_grad[:2])
-        gq = torch.empty(inp.shape, dtype=inp.dtype, device=inp.device) if need[0] else None
-        gkt = torch.empty(inp.shape, dtype=inp.dtype, device=inp.device) if need[1] else None
-        for idx in _slices(ctx.depth, inp.shape):
+        need = ctx.needs_input_grad
+        kt = other.transpose(-1, -2)
+        gq = _grad_like(inp) if need[0] else None
+        gkt = _grad_like(kt) if need[1] else None
+        if inp.numel():
+            x, y = _outer_addressable(inp, depth), _outer_addressable(kt, depth)
+            g, code = N.geometry(_lead(inp[(0,) * depth]), inp.shape[-2], inp.shape[-1], window_size), N.dtype_code(inp)
             if need[0] and need[1]:
-                window_matmul_backward(_v3(inp, idx), _v3(other, idx), window_size, _v3(grad_output, idx),
-                                       out=(_v3(gq, idx), _v3(gkt, idx)))
+                _outer_call(N.lib.wmm_window_bwd_outer, depth, (x, y, grad_output, gq, gkt),
+                            (N.operand, N.operand, _pointer, N.operand, N.operand), g, code)
             elif need[0]:
-                band_n(_v3(grad_output, idx), _addressable(_v3(other, idx).transpose(-1, -2)), window_size, out=_v3(gq, idx))
+                _outer_call(N.lib.wmm_band_n_outer, depth, (grad_output, y, gq), (_pointer, N.operand, N.operand), g, code)
             elif need[1]:
-                band_t(_v3(grad_output, idx), _addressable(_v3(inp, idx)), window_size, out=_v3(gkt, idx))
+                _outer_call(N.lib.wmm_band_t_outer, depth, (grad_output, x, gkt), (_pointer, N.operand, N.operand), g, code)
         return gq, (gkt.transpose(-1, -2) if need[1] else None), None, None
 
 
@@ -291,58 +327,82 @@ class _StridedUnwindowMatmulFunc(torch.autograd.Function):
     """UnwindowMatmulFunc for operands whose leading dimensions do not merge."""
 
     @staticmethod
-    @torch.amp.custom_fwd(device_type="cuda", cast_inputs=torch.float16)
     def forward(ctx, inp, other, window_size, depth):
+        inp, other = _autocast(inp, other)
         _require_cuda(inp, other)
         out = torch.empty(other.shape, dtype=other.dtype, device=other.device)
-        for idx in _slices(depth, other.shape):
-            unwindow_matmul_forward(_v3(inp, idx), _v3(other, idx), window_size, out=_v3(out, idx))
+        if out.numel():
+            a, v = _outer_band(inp, depth), _outer_addressable(other, depth)
+            g = N.geometry(_lead(other[(0,) * depth]), other.shape[-2], other.shape[-1], window_size)
+            _outer_call(N.lib.wmm_band_n_outer, depth, (a, v, out), (_pointer, N.operand, N.operand), g, N.dtype_code(other))
         ctx.save_for_backward(inp, other)
         ctx.depth = depth
         return out
 
     @staticmethod
-    @torch.amp.custom_bwd(device_type="cuda")
     def backward(ctx, grad_output):
         inp, other = ctx.saved_tensors
-        window_size = inp.shape[-1] // 2
-        need = tuple(ctx.needs_input_grad[:2])
+        depth, window_size = ctx.depth, inp.shape[-1] // 2
+        _require_cuda(inp, other, grad_output)
+        need = ctx.needs_input_grad
         ga = torch.empty(inp.shape, dtype=inp.dtype, device=inp.device) if need[0] else None
-        gv = torch.empty(other.shape, dtype=other.dtype, device=other.device) if need[1] else None
-        depth = max(ctx.depth, split_depth(grad_output))
-        for idx in _slices(depth, other.shape):
-            a3, v3, g3 = _v3(inp, idx), _v3(other, idx), _v3(grad_output, idx)
+        gv = _grad_like(other) if need[1] else None
+        if other.numel():
+            v, go = _outer_addressable(other, depth), _outer_addressable(grad_output, depth)
+            g, code = N.geometry(_lead(other[(0,) * depth]), other.shape[-2], other.shape[-1], window_size), N.dtype_code(other)
             if need[0] and need[1]:
-                unwindow_matmul_backward(a3, v3, window_size, g3, out=(_v3(ga, idx), _v3(gv, idx)))
+                _outer_call(N.lib.wmm_unwindow_bwd_outer, depth, (_outer_band(inp, depth), v, go, ga, gv),
+                            (_pointer, N.operand, N.operand, _pointer, N.operand), g, code)
             elif need[0]:
-                band_nt(_addressable(g3), _addressable(v3), window_size, out=_v3(ga, idx))
+                _outer_call(N.lib.wmm_band_nt_outer, depth, (go, v, ga), (N.operand, N.operand, _pointer), g, code)
             elif need[1]:
-                band_t(a3.contiguous(), _addressable(g3), window_size, out=_v3(gv, idx))
+                _outer_call(N.lib.wmm_band_t_outer, depth, (_outer_band(inp, depth), go, gv), (_pointer, N.operand, N.operand), g, code)
         return ga, gv, None, None
 
 
+def _pointer(t: torch.Tensor) -> int:
+    return t.data_ptr()
+
+
+def _outer_band(t: torch.Tensor, depth: int) -> torch.Tensor:
+    """A band whose slices below `depth` are contiguous."""
+    return t if t[(0,) * depth].is_contiguous() else t.contiguous()
+
+
 # ---- autograd nodes and the public functions ------------------------------------------------------
+# The leading dimensions are flattened inside the nodes: as reshapes outside, each would be one more node of the graph.
+
+
+def _merged(t: torch.Tensor) -> torch.Tensor:
+    return t if t.dim() == 3 else t.reshape(_lead(t), t.shape[-2], t.shape[-1])   # (an explicit size: -1 is ambiguous for empty tensors)
+
+
+def _merges(inp: torch.Tensor, other: torch.Tensor) -> bool:
+    """Whether both operands are 3-D views as they stand: the usual layouts, without trying (a transposed K is checked as stored)."""
+    return (inp.dim() == 3 or inp.is_contiguous()) and (other.dim() == 3 or other.is_contiguous() or other.transpose(-1, -2).is_contiguous())
 
 
 class WindowMatmulFunc(torch.autograd.Function):
     """window_matmul/window_matmul.py:7-27."""
 
     @staticmethod
-    @torch.amp.custom_fwd(device_type="cuda", cast_inputs=torch.float16)
     def forward(ctx, inp: torch.Tensor, other: torch.Tensor, window_size: int) -> torch.Tensor:
+        inp, other = _autocast(inp, other)
         _require_cuda(inp, other)
-        output = window_matmul_forward(inp, other, window_size)
+        output = window_matmul_forward(_merged(inp), _merged(other), window_size)
         ctx.save_for_backward(inp, other)
-        return output
+        return output if inp.dim() == 3 else output.view(*inp.shape[:-1], output.shape[-1])
 
     @staticmethod
-    @torch.amp.custom_bwd(device_type="cuda")
     def backward(ctx, grad_output: torch.Tensor) -> Tuple[Optional[torch.Tensor], Optional[torch.Tensor], None]:
         window_size = (grad_output.shape[-1]) // 2
         inp, other = ctx.saved_tensors
         inp_grad, other_grad = window_matmul_backward(
-            inp, other, window_size, grad_output, need=tuple(ctx.needs_input_grad[:2])
+            _merged(inp), _merged(other), window_size, _merged(grad_output), need=ctx.needs_input_grad[:2]
         )
+        if inp.dim() != 3:
+            inp_grad = None if inp_grad is None else inp_grad.view(inp.shape)
+            other_grad = None if other_grad is None else other_grad.transpose(-1, -2).view(inp.shape).transpose(-1, -2)
         return inp_grad, other_grad, None
 
 
@@ -351,9 +411,11 @@ def window_matmul(inp: torch.Tensor, other: torch.Tensor, window_size: int) -> t
     if not window_size:
         return (inp * other.transpose(-1, -2)).sum(dim=-1, keepdim=True)
     *dims, seq_len, hidden_dim = inp.shape
-    if inp.is_cuda and other.is_cuda and other.shape == (*dims, hidden_dim, seq_len):
-        depth = split_depth(inp, other)
-        if depth:   # leading dimensions that do not merge: no copy, one call per outer index
+    if dims and other.shape == (*dims, hidden_dim, seq_len):
+        if _merges(inp, other):
+            return WindowMatmulFunc.apply(inp, other, window_size)
+        depth = split_depth(inp, other) if inp.is_cuda and other.is_cuda else 0
+        if depth:   # leading dimensions that do not merge: no copy, one launch per outer index
             return _StridedWindowMatmulFunc.apply(inp, other, window_size, depth)
     inp = inp.reshape(_lead(inp), seq_len, hidden_dim)        # (-1 would be ambiguous for an empty sequence)
     other = other.reshape(_lead(other), hidden_dim, seq_len)
@@ -366,21 +428,23 @@ class UnwindowMatmulFunc(torch.autograd.Function):
     """window_matmul/window_matmul.py:43-63."""
 
     @staticmethod
-    @torch.amp.custom_fwd(device_type="cuda", cast_inputs=torch.float16)
     def forward(ctx, inp: torch.Tensor, other: torch.Tensor, window_size: int) -> torch.Tensor:
+        inp, other = _autocast(inp, other)
         _require_cuda(inp, other)
-        output = unwindow_matmul_forward(inp, other, window_size)
+        output = unwindow_matmul_forward(_merged(inp), _merged(other), window_size)
         ctx.save_for_backward(inp, other)
-        return output
+        return output if other.dim() == 3 else output.view(other.shape)
 
     @staticmethod
-    @torch.amp.custom_bwd(device_type="cuda")
     def backward(ctx, grad_output: torch.Tensor) -> Tuple[Optional[torch.Tensor], Optional[torch.Tensor], None]:
         inp, other = ctx.saved_tensors
         window_size = (inp.shape[-1]) // 2
         inp_grad, other_grad = unwindow_matmul_backward(
-            inp, other, window_size, grad_output, need=tuple(ctx.needs_input_grad[:2])
+            _merged(inp), _merged(other), window_size, _merged(grad_output), need=ctx.needs_input_grad[:2]
         )
+        if other.dim() != 3:
+            inp_grad = None if inp_grad is None else inp_grad.view(inp.shape)
+            other_grad = None if other_grad is None else other_grad.view(other.shape)
         return inp_grad, other_grad, None
 
 
@@ -389,8 +453,10 @@ def unwindow_matmul(inp: torch.Tensor, other: torch.Tensor, window_size: int) ->
     if not window_size:
         return inp * other
     *dims, seq_len, hidden_dim = other.shape
-    if inp.is_cuda and other.is_cuda and inp.shape == (*dims, seq_len, window_size * 2 + 1):
-        depth = split_depth(inp, other)
+    if dims and inp.shape == (*dims, seq_len, window_size * 2 + 1):
+        if _merges(inp, other):
+            return UnwindowMatmulFunc.apply(inp, other, window_size)
+        depth = split_depth(inp, other) if inp.is_cuda and other.is_cuda else 0
         if depth:
             return _StridedUnwindowMatmulFunc.apply(inp, other, window_size, depth)
     inp = inp.reshape(_lead(inp), seq_len, window_size * 2 + 1)

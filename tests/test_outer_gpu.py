@@ -1,0 +1,78 @@
+"""Operands whose batch dimensions do not merge: the calls that walk the outermost dimension in the library."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _views(B, H, M, N, dtype, how, g):
+    """A (B, H, M, N) operand at its place in a larger tensor, as a leaf and its view."""
+    if how == "projection":
+        leaf = torch.randn(B, M, H * N, device="cuda", generator=g).to(dtype).requires_grad_(True)
+        return leaf, leaf.view(B, M, H, N).transpose(1, 2)
+    if how == "fused":        # one third of a (B, M, 3, H, N) projection
+        leaf = torch.randn(B, M, 3, H, N, device="cuda", generator=g).to(dtype).requires_grad_(True)
+        return leaf, leaf[:, :, 1].transpose(1, 2)
+    if how == "deep":         # five dimensions, two of which do not merge with the next
+        leaf = torch.randn(H, M, B, 1, N, device="cuda", generator=g).to(dtype).requires_grad_(True)
+        return leaf, leaf.permute(2, 0, 3, 1, 4)
+    leaf = torch.randn(H, B, N, M, device="cuda", generator=g).to(dtype).requires_grad_(True)   # "position": hidden rows of positions
+    return leaf, leaf.permute(1, 0, 3, 2)
+
+
+@pytest.mark.parametrize("how", ["projection", "fused", "deep", "position"])
+@pytest.mark.parametrize("dtype,N", [(torch.bfloat16, 64), (torch.float16, 20), (torch.float32, 20), (torch.float32, 33)])
+@pytest.mark.parametrize("need", [(True, True, True), (True, False, False), (False, True, True)])
+def test_strided_operands_give_the_results_of_copies(how, dtype, N, need):
+    """Both operators, forward and backward, bit for bit what contiguous copies give, whichever gradients are asked for."""
+    from window_matmul import _native, unwindow_matmul, window_matmul
+
+    B, H, M, w = 3, 2, 72, 12
+    g = torch.Generator(device="cuda")
+    g.manual_seed(2)
+    made = [_views(B, H, M, N, dtype, how, g) for _ in range(3)]
+    go = torch.randn(made[0][1].shape, device="cuda", generator=g).to(dtype)
+    wanted = [leaf for (leaf, _), n in zip(made, need) if n]
+    for (leaf, _), n in zip(made, need):
+        leaf.requires_grad_(n)
+
+    def run(copy):
+        q, k, v = (_regrow(leaf, how) for leaf, _ in made)
+        if copy:
+            q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
+        a = window_matmul(q, k.transpose(-1, -2), w)
+        o = unwindow_matmul(a, v, w)
+        return [a.detach(), o.detach()] + list(torch.autograd.grad(o, wanted, go))
+
+    def _regrow(leaf, how):
+        if how == "projection":
+            return leaf.view(B, M, H, N).transpose(1, 2)
+        if how == "fused":
+            return leaf[:, :, 1].transpose(1, 2)
+        return leaf.permute(2, 0, 3, 1, 4) if how == "deep" else leaf.permute(1, 0, 3, 2)
+
+    for got, want in zip(run(False), run(True)):
+        assert got.shape == want.shape
+        # a position-major operand may take another kernel than its copy: one rounding of the 16-bit type apart
+        if how == "position" and dtype != torch.float32:
+            assert (got.double() - want.double()).norm() <= 1e-2 * want.double().norm()
+        else:
+            assert torch.equal(got, want)
+    assert _native.device_status() == 0
+
+
+def test_autocast_is_the_cast_of_the_inputs():
+    """Under autocast both operators compute in float16 and hand float32 gradients to float32 leaves; outside nothing is cast."""
+    from window_matmul import unwindow_matmul, window_matmul
+
+    q, k, v = (torch.randn(2, 3, 40, 16, device="cuda").requires_grad_(True) for _ in range(3))
+    with torch.autocast("cuda"):
+        a = window_matmul(q, k.transpose(-1, -2), 5)
+        o = unwindow_matmul(a, v, 5)
+    assert a.dtype == torch.float16 and o.dtype == torch.float16 and a.shape == (2, 3, 40, 11)
+    grads = torch.autograd.grad(o, (q, k, v), torch.ones_like(o))
+    h = [t.detach().half().requires_grad_(True) for t in (q, k, v)]
+    o2 = unwindow_matmul(window_matmul(h[0], h[1].transpose(-1, -2), 5), h[2], 5)
+    assert torch.equal(o, o2)
+    for x, y in zip(grads, torch.autograd.grad(o2, h, torch.ones_like(o2))):
+        assert x.dtype == torch.float32 and torch.equal(x, y.float())
