@@ -145,8 +145,8 @@ WMM_API int wmm_set_cta_limits(int contraction_ctas, int exchange_ctas);
 WMM_API int64_t wmm_device_status(int clear);
 /* The five compute calls over operands whose batch dimensions do not merge into one stride (the (B, H, M, N) view of a
  * (B, M, H*N) projection): `outer` calls of the function without the suffix, the i-th with every tensor moved on by i times
- * its entry of `strides` (elements, in the order of the arguments), on `stream` one after another.  `g` describes one of
- * them.  The first status that is not WMM_OK ends the call.  (The reference copies such operands together,
+ * its entry of `strides` (elements, in the order of the arguments).  `g` describes one of them.  The calls may overlap on the
+ * device: outputs must not share memory with inputs or with each other.  The first status that is not WMM_OK ends the call.  (The reference copies such operands together,
  * window_matmul/window_matmul.py:36-37,72-73.) */
 WMM_API int wmm_band_nt_outer(const wmm_operand *x, const wmm_operand *y, void *band, int outer, const int64_t strides[3],
                               const wmm_geometry *g, int dtype, unsigned flags, void *stream);

@@ -122,7 +122,18 @@ int pick_family(wmm::Primitive prim, const wmm::Problem &p) {
 
 bool wants_tensor(wmm::Primitive prim, const wmm::Problem &p) { return pick_family(prim, p) == 1; }
 
-int dispatch(wmm::Primitive prim, const wmm::Problem &p, void *stream) {
+// The launches of one call that depend on none of the others (see griddep_enter in wmm_ptx.cuh): the first one, then the rest.
+struct Chain {
+  bool started = false;
+  int next() {
+    const int place = started ? 1 : 2;   // CHAIN_LATE_WAIT, CHAIN_FIRST
+    started = true;
+    return place;
+  }
+};
+
+int dispatch(wmm::Primitive prim, wmm::Problem &p, void *stream, Chain *chain = nullptr) {
+  p.chain = chain ? chain->next() : 0;
   const int family = pick_family(prim, p);
   if (family == 0 && (p.flags & WMM_FLAG_REQUIRE_TENSOR))
     return fail(WMM_ERR_UNSUPPORTED, "no tensor-core kernel takes this problem (primitive %d)", (int)prim);
@@ -364,28 +375,42 @@ int wmm_query_path(int primitive, const wmm_operand *a, const wmm_operand *b, co
   return pick_family((wmm::Primitive)primitive, p);
 }
 
-int wmm_band_nt(const wmm_operand *x, const wmm_operand *y, void *band, const wmm_geometry *g, int dtype,
-                unsigned flags, void *stream) {
+static int run_band_nt(const wmm_operand *x, const wmm_operand *y, void *band, const wmm_geometry *g, int dtype, unsigned flags,
+                       void *stream, Chain *chain) {
   wmm::Problem p{};
   const int s = build(wmm::BAND_NT, p, x, y, nullptr, band, nullptr, g, dtype, flags);
   if (s != WMM_OK) return s < 0 ? s : WMM_OK;
-  return dispatch(wmm::BAND_NT, p, stream);
+  return dispatch(wmm::BAND_NT, p, stream, chain);
 }
 
-int wmm_band_n(const void *band, const wmm_operand *y, const wmm_operand *out, const wmm_geometry *g, int dtype,
-               unsigned flags, void *stream) {
+static int run_band_n(const void *band, const wmm_operand *y, const wmm_operand *out, const wmm_geometry *g, int dtype,
+                      unsigned flags, void *stream, Chain *chain) {
   wmm::Problem p{};
   const int s = build(wmm::BAND_N, p, nullptr, y, band, nullptr, out, g, dtype, flags);
   if (s != WMM_OK) return s < 0 ? s : WMM_OK;
-  return dispatch(wmm::BAND_N, p, stream);
+  return dispatch(wmm::BAND_N, p, stream, chain);
 }
 
-int wmm_band_t(const void *band, const wmm_operand *x, const wmm_operand *out, const wmm_geometry *g, int dtype,
-               unsigned flags, void *stream) {
+static int run_band_t(const void *band, const wmm_operand *x, const wmm_operand *out, const wmm_geometry *g, int dtype,
+                      unsigned flags, void *stream, Chain *chain) {
   wmm::Problem p{};
   const int s = build(wmm::BAND_T, p, x, nullptr, band, nullptr, out, g, dtype, flags);
   if (s != WMM_OK) return s < 0 ? s : WMM_OK;
-  return dispatch(wmm::BAND_T, p, stream);
+  return dispatch(wmm::BAND_T, p, stream, chain);
+}
+
+int wmm_band_nt(const wmm_operand *x, const wmm_operand *y, void *band, const wmm_geometry *g, int dtype, unsigned flags, void *stream) {
+  return run_band_nt(x, y, band, g, dtype, flags, stream, nullptr);
+}
+
+int wmm_band_n(const void *band, const wmm_operand *y, const wmm_operand *out, const wmm_geometry *g, int dtype, unsigned flags,
+               void *stream) {
+  return run_band_n(band, y, out, g, dtype, flags, stream, nullptr);
+}
+
+int wmm_band_t(const void *band, const wmm_operand *x, const wmm_operand *out, const wmm_geometry *g, int dtype, unsigned flags,
+               void *stream) {
+  return run_band_t(band, x, out, g, dtype, flags, stream, nullptr);
 }
 
 int wmm_band_t_edges(const void *band, const wmm_operand *x, const wmm_operand *out, float *edges, int edge_rows,
@@ -406,8 +431,8 @@ int wmm_band_t_edges(const void *band, const wmm_operand *x, const wmm_operand *
   return dispatch(wmm::BAND_T, p, stream);
 }
 
-int wmm_window_bwd(const wmm_operand *q, const wmm_operand *kt, const void *grad_band, const wmm_operand *grad_q,
-                   const wmm_operand *grad_kt, const wmm_geometry *g, int dtype, unsigned flags, void *stream) {
+static int run_window_bwd(const wmm_operand *q, const wmm_operand *kt, const void *grad_band, const wmm_operand *grad_q,
+                   const wmm_operand *grad_kt, const wmm_geometry *g, int dtype, unsigned flags, void *stream, Chain *chain) {
   if (int s = plain_geometry(g)) return s;
   // validate both halves before launching either, so a bad argument never leaves half a result
   wmm::Problem pq{}, pk{};
@@ -419,6 +444,7 @@ int wmm_window_bwd(const wmm_operand *q, const wmm_operand *kt, const void *grad
       wmm::tensor_fused_pair_eligible(pq, pk)) {
     // both passes over grad_A in one launch: the band is read from HBM once
     int launches = 0;
+    pq.chain = chain ? chain->next() : 0;
     cudaError_t e = wmm::launch_tensor_fused_pair(pq, pk, (cudaStream_t)stream, &launches);
     g_launches.fetch_add((uint64_t)launches, std::memory_order_relaxed);
     if (e != cudaSuccess)
@@ -426,14 +452,14 @@ int wmm_window_bwd(const wmm_operand *q, const wmm_operand *kt, const void *grad
     return WMM_OK;
   }
   if (sq == WMM_OK)
-    if (int s = dispatch(wmm::BAND_N, pq, stream)) return s;
+    if (int s = dispatch(wmm::BAND_N, pq, stream, chain)) return s;
   if (sk == WMM_OK)
-    if (int s = dispatch(wmm::BAND_T, pk, stream)) return s;
+    if (int s = dispatch(wmm::BAND_T, pk, stream, chain)) return s;
   return WMM_OK;
 }
 
-int wmm_unwindow_bwd(const void *band, const wmm_operand *v, const wmm_operand *grad_o, void *grad_band,
-                     const wmm_operand *grad_v, const wmm_geometry *g, int dtype, unsigned flags, void *stream) {
+static int run_unwindow_bwd(const void *band, const wmm_operand *v, const wmm_operand *grad_o, void *grad_band,
+                     const wmm_operand *grad_v, const wmm_geometry *g, int dtype, unsigned flags, void *stream, Chain *chain) {
   if (int s = plain_geometry(g)) return s;
   wmm::Problem pa{}, pv{};
   const int sa = build(wmm::BAND_NT, pa, grad_o, v, nullptr, grad_band, nullptr, g, dtype, flags);
@@ -441,10 +467,20 @@ int wmm_unwindow_bwd(const void *band, const wmm_operand *v, const wmm_operand *
   const int sv = build(wmm::BAND_T, pv, grad_o, nullptr, band, nullptr, grad_v, g, dtype, flags);
   if (sv < 0) return sv;
   if (sa == WMM_OK)
-    if (int s = dispatch(wmm::BAND_NT, pa, stream)) return s;
+    if (int s = dispatch(wmm::BAND_NT, pa, stream, chain)) return s;
   if (sv == WMM_OK)
-    if (int s = dispatch(wmm::BAND_T, pv, stream)) return s;
+    if (int s = dispatch(wmm::BAND_T, pv, stream, chain)) return s;
   return WMM_OK;
+}
+
+int wmm_window_bwd(const wmm_operand *q, const wmm_operand *kt, const void *grad_band, const wmm_operand *grad_q,
+                   const wmm_operand *grad_kt, const wmm_geometry *g, int dtype, unsigned flags, void *stream) {
+  return run_window_bwd(q, kt, grad_band, grad_q, grad_kt, g, dtype, flags, stream, nullptr);
+}
+
+int wmm_unwindow_bwd(const void *band, const wmm_operand *v, const wmm_operand *grad_o, void *grad_band,
+                     const wmm_operand *grad_v, const wmm_geometry *g, int dtype, unsigned flags, void *stream) {
+  return run_unwindow_bwd(band, v, grad_o, grad_band, grad_v, g, dtype, flags, stream, nullptr);
 }
 
 // ---- one call per outer index (see include/wmm_b200.h) ----
@@ -467,9 +503,10 @@ int wmm_band_nt_outer(const wmm_operand *x, const wmm_operand *y, void *band, in
   if (int s = outer_ok(outer, strides)) return s;
   if (!x || !y) return fail(WMM_ERR_NULL, "an operand is NULL");
   const int64_t e = (int64_t)elem_size(dtype);
+  Chain chain, *c = outer > 1 ? &chain : nullptr;
   for (int64_t i = 0; i < outer; ++i) {
     const wmm_operand xi = shifted_op(x, i * strides[0] * e), yi = shifted_op(y, i * strides[1] * e);
-    if (int s = wmm_band_nt(&xi, &yi, shifted_out(band, i * strides[2] * e), g, dtype, flags, stream)) return s;
+    if (int s = run_band_nt(&xi, &yi, shifted_out(band, i * strides[2] * e), g, dtype, flags, stream, c)) return s;
   }
   return WMM_OK;
 }
@@ -479,9 +516,10 @@ int wmm_band_n_outer(const void *band, const wmm_operand *y, const wmm_operand *
   if (int s = outer_ok(outer, strides)) return s;
   if (!y || !out) return fail(WMM_ERR_NULL, "an operand is NULL");
   const int64_t e = (int64_t)elem_size(dtype);
+  Chain chain, *c = outer > 1 ? &chain : nullptr;
   for (int64_t i = 0; i < outer; ++i) {
     const wmm_operand yi = shifted_op(y, i * strides[1] * e), oi = shifted_op(out, i * strides[2] * e);
-    if (int s = wmm_band_n(shifted_in(band, i * strides[0] * e), &yi, &oi, g, dtype, flags, stream)) return s;
+    if (int s = run_band_n(shifted_in(band, i * strides[0] * e), &yi, &oi, g, dtype, flags, stream, c)) return s;
   }
   return WMM_OK;
 }
@@ -491,9 +529,10 @@ int wmm_band_t_outer(const void *band, const wmm_operand *x, const wmm_operand *
   if (int s = outer_ok(outer, strides)) return s;
   if (!x || !out) return fail(WMM_ERR_NULL, "an operand is NULL");
   const int64_t e = (int64_t)elem_size(dtype);
+  Chain chain, *c = outer > 1 ? &chain : nullptr;
   for (int64_t i = 0; i < outer; ++i) {
     const wmm_operand xi = shifted_op(x, i * strides[1] * e), oi = shifted_op(out, i * strides[2] * e);
-    if (int s = wmm_band_t(shifted_in(band, i * strides[0] * e), &xi, &oi, g, dtype, flags, stream)) return s;
+    if (int s = run_band_t(shifted_in(band, i * strides[0] * e), &xi, &oi, g, dtype, flags, stream, c)) return s;
   }
   return WMM_OK;
 }
@@ -504,10 +543,11 @@ int wmm_window_bwd_outer(const wmm_operand *q, const wmm_operand *kt, const void
   if (int s = outer_ok(outer, strides)) return s;
   if (!q || !kt || !grad_q || !grad_kt) return fail(WMM_ERR_NULL, "an operand is NULL");
   const int64_t e = (int64_t)elem_size(dtype);
+  Chain chain, *c = outer > 1 ? &chain : nullptr;
   for (int64_t i = 0; i < outer; ++i) {
     const wmm_operand qi = shifted_op(q, i * strides[0] * e), ki = shifted_op(kt, i * strides[1] * e);
     const wmm_operand gqi = shifted_op(grad_q, i * strides[3] * e), gki = shifted_op(grad_kt, i * strides[4] * e);
-    if (int s = wmm_window_bwd(&qi, &ki, shifted_in(grad_band, i * strides[2] * e), &gqi, &gki, g, dtype, flags, stream)) return s;
+    if (int s = run_window_bwd(&qi, &ki, shifted_in(grad_band, i * strides[2] * e), &gqi, &gki, g, dtype, flags, stream, c)) return s;
   }
   return WMM_OK;
 }
@@ -518,10 +558,11 @@ int wmm_unwindow_bwd_outer(const void *band, const wmm_operand *v, const wmm_ope
   if (int s = outer_ok(outer, strides)) return s;
   if (!v || !grad_o || !grad_v) return fail(WMM_ERR_NULL, "an operand is NULL");
   const int64_t e = (int64_t)elem_size(dtype);
+  Chain chain, *c = outer > 1 ? &chain : nullptr;
   for (int64_t i = 0; i < outer; ++i) {
     const wmm_operand vi = shifted_op(v, i * strides[1] * e), goi = shifted_op(grad_o, i * strides[2] * e);
     const wmm_operand gvi = shifted_op(grad_v, i * strides[4] * e);
-    if (int s = wmm_unwindow_bwd(shifted_in(band, i * strides[0] * e), &vi, &goi, shifted_out(grad_band, i * strides[3] * e), &gvi, g, dtype, flags, stream))
+    if (int s = run_unwindow_bwd(shifted_in(band, i * strides[0] * e), &vi, &goi, shifted_out(grad_band, i * strides[3] * e), &gvi, g, dtype, flags, stream, c))
       return s;
   }
   return WMM_OK;

@@ -30,6 +30,7 @@ struct Problem {
   // end) once more, unrounded, as fp32 rows of a (B, 2 * edge_rows, N) contiguous buffer; NULL = none
   float *edges;
   int32_t edge_rows, edge_skip;
+  int32_t chain;   // place in a chain of independent launches: 0 none, else the bits of wmm_ptx.cuh (tensor-core families)
 };
 
 enum Primitive { BAND_NT = 1, BAND_N = 2, BAND_T = 3 };

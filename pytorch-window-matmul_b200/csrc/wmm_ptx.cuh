@@ -121,6 +121,28 @@ __device__ __forceinline__ void named_bar_sync(uint32_t id, uint32_t threads) {
 // before it may touch global memory that the predecessor reads or writes.  Both are no-ops in a plain launch.
 __device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// A chain of launches that neither read nor overwrite what the others write (the slices of an operand whose batch dimensions do
+// not merge) may run into one another.  Its first kernel waits for the predecessor of the chain BEFORE it lets the second be
+// scheduled, so every later kernel of the chain finds that predecessor complete when it starts and does its waiting (for
+// the kernel before it) last: it is complete only after the whole chain up to it, which is what the successor waits for.
+// A slice that leaves SMs idle (4 x 12 heads of 2048 rows: 192 row tiles a slice on 148 SMs) thereby shares them with the next one:
+// the five contractions forward and backward over such views take 217 us of device time instead of 258 (N = 64, w = 256);
+// 16 x 12 x 512 rows, w = 128: 354 instead of 484; 32 x 8 x 500 rows, w = 100: 832 instead of 1425.
+enum { CHAIN_LATE_WAIT = 1, CHAIN_FIRST = 2 };
+__device__ __forceinline__ void griddep_enter(int chain) {
+  if (chain & CHAIN_LATE_WAIT) {
+    griddep_launch_dependents();
+  } else if (chain & CHAIN_FIRST) {
+    griddep_wait();
+    griddep_launch_dependents();
+  } else {
+    griddep_launch_dependents();
+    griddep_wait();
+  }
+}
+__device__ __forceinline__ void griddep_leave(int chain) {
+  if (chain & CHAIN_LATE_WAIT) griddep_wait();
+}
 
 // ---- TMA ------------------------------------------------------------------------------------------
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap *m) {

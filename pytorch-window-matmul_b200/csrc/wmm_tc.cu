@@ -310,6 +310,7 @@ template <int ET, int NH, bool YMN, bool PAIRED> cudaError_t launch_nt(const Pro
   k.B = p.B; k.M = p.M; k.w = p.w; k.off = p.off; k.lo = p.lo; k.hi = p.hi;
   k.tiles_per_batch = (p.M + TILE - 1) / TILE;
   k.total_tiles = k.tiles_per_batch * p.B;
+  k.chain = p.chain;
   k.nchunks = (TILE + 2 * p.w + CHUNK - 1) / CHUNK;
   k.paired = PAIRED ? 1 : 0;
   k.band = p.o;
@@ -361,6 +362,7 @@ template <bool BF16, int NH, int MODE, bool YMN> cudaError_t launch_mm(const Pro
   k.B = p.B; k.M = p.M; k.Mo = p.Mo; k.w = p.w; k.off = p.off; k.lo = p.lo; k.hi = p.hi;
   k.tiles_per_batch = (out_rows + TILE - 1) / TILE;
   k.total_tiles = k.tiles_per_batch * p.B;
+  k.chain = p.chain;
   k.nchunks = (TILE + 2 * p.w + 127) / 128;
   k.edges = MODE == 1 ? p.edges : nullptr;
   k.edge_rows = MODE == 1 ? p.edge_rows : 0;
@@ -412,6 +414,7 @@ template <int NH, bool TR> cudaError_t launch_mm32(const Problem &p, cudaStream_
   k.B = p.B; k.M = p.M; k.Mo = p.Mo; k.w = p.w; k.off = p.off; k.lo = p.lo; k.hi = p.hi;
   k.tiles_per_batch = (out_rows + TILE - 1) / TILE;
   k.total_tiles = k.tiles_per_batch * p.B;
+  k.chain = p.chain;
   k.nchunks = (TILE + 2 * p.w + M32_RC - 1) / M32_RC;
   auto kern = band_mm_tf32_kernel<NH, TR>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::ALLOC);
@@ -455,6 +458,7 @@ template <bool BF16, int NH> cudaError_t launch_sweep(const Problem &pn, const P
   k.B = pn.B; k.M = pn.M; k.w = pn.w; k.D = pn.w / 128;
   k.T = (pn.M + TILE - 1) / TILE;
   k.total_rows = k.B * k.T;
+  k.chain = pn.chain;
   auto kern = band_bwd_sweep_kernel<BF16, NH>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::ALLOC);
   if (e != cudaSuccess) {
@@ -498,6 +502,7 @@ void fill_ragged(RagParams &k, const Problem &p, int rows) {
   k.B = p.B; k.M = p.M; k.N = p.N; k.w = p.w; k.Mo = p.Mo; k.off = p.off; k.lo = p.lo; k.hi = p.hi;
   k.tiles_per_batch = (rows + TILE - 1) / TILE;
   k.total_tiles = k.tiles_per_batch * p.B;
+  k.chain = p.chain;
   k.parts = k.part_chunks = 1;
   k.a_mode = row_mode(p.a, p.a_sb, p.a_sr, p.N, p.B);   // (band_nt)
   k.b_mode = operand_mode(p.b, p.b_sb, p.b_sr, p.b_sc, p.N, p.B);

@@ -26,6 +26,7 @@ constexpr unsigned long long ST_MM_TIMEOUT = 1ull << 1;
 struct MmParams {
   int B, M, Mo, w, off, lo, hi;
   int tiles_per_batch, total_tiles, nchunks;
+  int chain;   // see griddep_enter
   // band_t (MODE 1) only: unrounded fp32 copy of output rows [edge_skip, edge_rows) and [Mo - edge_rows, Mo - edge_skip)
   // of every batch entry, at the same row index of a (B, 2 * edge_rows, NH) contiguous buffer (row Mo - edge_rows is its
   // row edge_rows), for a sequence shard whose edge rows are summed with a neighbour's
@@ -100,8 +101,7 @@ band_mm_tc_kernel(const __grid_constant__ CUtensorMap map_band, const __grid_con
   const uint32_t tmem_base = *tmem_slot;
   // Everything above (barriers, tensor memory, tensor-map prefetch) may run under the tail of the previous kernel of the
   // stream; from here on global memory is read and written.
-  griddep_launch_dependents();
-  griddep_wait();
+  griddep_enter(p.chain);
 
   // Work items, identical in every role: item -> (tile, transposed?).
   const int total_items = MODE == 2 ? 2 * p.total_tiles : p.total_tiles;
@@ -360,6 +360,7 @@ band_mm_tc_kernel(const __grid_constant__ CUtensorMap map_band, const __grid_con
   }
 
   // ---------------- teardown ----------------
+  griddep_leave(p.chain);
   tc_fence_before_sync();
   __syncthreads();
   if (*abort_flag) {

@@ -77,8 +77,7 @@ band_mm_tf32_kernel(const __grid_constant__ CUtensorMap map_band, const __grid_c
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  griddep_launch_dependents();
-  griddep_wait();
+  griddep_enter(p.chain);
 
   // Tile / chunk geometry.  t0 = first row (band_n) or position (band_t) of the tile; chunk c covers 64 steps of the
   // reduction:
@@ -281,6 +280,7 @@ band_mm_tf32_kernel(const __grid_constant__ CUtensorMap map_band, const __grid_c
   }
 
   // ---------------- teardown ----------------
+  griddep_leave(p.chain);
   tc_fence_before_sync();
   __syncthreads();
   if (*abort_flag) {

@@ -30,6 +30,7 @@ constexpr unsigned long long ST_NT_TIMEOUT = 1ull << 0;
 struct NtParams {
   int B, M, w, off, lo, hi;
   int tiles_per_batch, total_tiles, nchunks;
+  int chain;   // see griddep_enter
   int paired;  // 2w is a multiple of 128: merge first and last chunk of a tile
   void *band;
   int64_t band_sb;   // elements between batch entries of the band (rows written without TMA)
@@ -159,8 +160,7 @@ band_nt_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   // Everything above (barriers, tensor memory, tensor-map prefetch) may run under the tail of the previous kernel of the
   // stream; from here on global memory is read and written.
   if (threadIdx.x == 0) WMM_TRACE_POINT(1);
-  griddep_launch_dependents();
-  griddep_wait();
+  griddep_enter(p.chain);
   if (threadIdx.x == 0) WMM_TRACE_POINT(2);
 
   if (warp == 0) {
@@ -585,6 +585,7 @@ band_nt_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   }
 
   // ---------------- teardown ----------------
+  griddep_leave(p.chain);
   tc_fence_before_sync();
   __syncthreads();
   if (*abort_flag) {

@@ -39,6 +39,7 @@ struct RagParams {
   int tiles_per_batch, total_tiles;
   int parts, part_chunks;    // band_nt: a row tile's chunks are shared by `parts` work items of part_chunks each
   int a_mode, b_mode, o_mode;
+  int chain;                 // see griddep_enter
 };
 
 // word `lane` of line `row` in a tile of 128-byte lines with the 128-byte swizzle
@@ -218,8 +219,7 @@ __global__ void __launch_bounds__(RMM_THREADS, 1) band_mm_ragged_kernel(const Ra
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  griddep_launch_dependents();
-  griddep_wait();
+  griddep_enter(p.chain);
 
   const int W = 2 * p.w + 1;
   if (warp >= 4 && warp < 20) {
@@ -397,6 +397,7 @@ __global__ void __launch_bounds__(RMM_THREADS, 1) band_mm_ragged_kernel(const Ra
     }
   }
 
+  griddep_leave(p.chain);
   tc_fence_before_sync();
   __syncthreads();
   if (*abort_flag) {   // let the MMAs in flight end before tensor memory and shared memory go
@@ -462,8 +463,7 @@ __global__ void __launch_bounds__(RNT_THREADS, 1) band_nt_ragged_kernel(const Ra
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  griddep_launch_dependents();
-  griddep_wait();
+  griddep_enter(p.chain);
 
   const int W = 2 * p.w + 1;
   auto tile_at = [&](int item, int &b, int &r0, int &delta, int &c0, int &c1) {   // its chunks are c0 .. c1-1
@@ -608,6 +608,7 @@ __global__ void __launch_bounds__(RNT_THREADS, 1) band_nt_ragged_kernel(const Ra
     }
   }
 
+  griddep_leave(p.chain);
   tc_fence_before_sync();
   __syncthreads();
   if (*abort_flag) {   // let the MMAs in flight end before tensor memory and shared memory go

@@ -27,6 +27,7 @@ constexpr unsigned long long ST_SWEEP_TIMEOUT = 1ull << 4;
 struct SweepParams {
   int B, M, w, D, T;   // T = row tiles (= position tiles) per sequence
   int total_rows;      // B * T
+  int chain;           // see griddep_enter
   // outputs (element strides; unit column stride): written straight from registers, a 2 NH-byte row per thread
   uint16_t *gq, *gk;
   int64_t gq_sb, gq_sr, gk_sb, gk_sr;
@@ -147,8 +148,7 @@ band_bwd_sweep_kernel(const __grid_constant__ CUtensorMap map_band, const __grid
   const uint32_t tmem_base = *tmem_slot;
   // Everything above (barriers, tensor memory, tensor-map prefetch) may run under the tail of the previous kernel of the
   // stream; from here on global memory is read and written.
-  griddep_launch_dependents();
-  griddep_wait();
+  griddep_enter(p.chain);
   // tensor memory columns: row accumulators at 0 and NH, column slot s at (2 + s) NH
   auto tmem_row = [&](int as) { return tmem_base + (uint32_t)(as * NH); };
   auto tmem_col = [&](int slot) { return tmem_base + (uint32_t)((2 + slot) * NH); };
@@ -397,6 +397,7 @@ band_bwd_sweep_kernel(const __grid_constant__ CUtensorMap map_band, const __grid
   }
 
   // ---------------- teardown ----------------
+  griddep_leave(p.chain);
   tc_fence_before_sync();
   __syncthreads();
   if (*abort_flag) {

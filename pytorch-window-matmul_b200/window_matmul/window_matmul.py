@@ -268,19 +268,30 @@ def _grad_like(t: torch.Tensor) -> torch.Tensor:
     return torch.empty(t.shape, dtype=t.dtype, device=t.device)
 
 
-def _outer_call(call, depth: int, tensors, pack, geometry, code) -> None:
+def _outer_call(call, depth: int, tensors, geometry, code) -> None:
     """call(...) for every outer index of the first `depth` dimensions, the innermost of them walked by the library.
-    `tensors` in the order of the call's arguments; pack[i] makes the argument of tensors[i]."""
-    lead = tensors[0].shape[:depth]
-    strides = (N.ctypes.c_int64 * len(tensors))(*[t.stride(depth - 1) for t in tensors])
-    for idx in _slices(depth - 1, lead):
-        first = [_v3(t[idx + (0,)], ()) for t in tensors]
-        N.run(call, first[0], *[p(t) for p, t in zip(pack, first)], lead[-1], strides, geometry, code, _FLAGS)
+    `tensors` in the order of the call's arguments: operands as (view, True), bands as (view, False)."""
+    ref = tensors[0][0]
+    strides = (N.ctypes.c_int64 * len(tensors))(*[t.stride(depth - 1) for t, _ in tensors])
+    for idx in _slices(depth - 1, ref.shape) if depth > 1 else ((),):
+        args = []
+        for t, operand in tensors:
+            if idx:
+                t = t[idx]
+            if not operand:
+                args.append(t.data_ptr())
+            elif ref.dim() == depth + 3:      # what is left of the leading dimensions is the batch, as it stands
+                args.append(N.Operand(t.data_ptr(), *t.stride()[-3:]))
+            else:
+                args.append(N.operand(_v3(t[0], ())))
+        N.run(call, ref, *args, ref.shape[depth - 1], strides, geometry, code, _FLAGS)
 
 
 def _outer_addressable(t: torch.Tensor, depth: int) -> torch.Tensor:
     """An operand whose slices below `depth` are (batch, rows, cols) views the kernels can address well."""
-    return t if (t.stride(-1) == 1 or t.stride(-2) == 1) and _viewable3(t[(0,) * depth]) else t.contiguous()
+    if t.stride(-1) != 1 and t.stride(-2) != 1:
+        return t.contiguous()
+    return t if t.dim() == depth + 3 or _viewable3(t[(0,) * depth]) else t.contiguous()
 
 
 class _StridedWindowMatmulFunc(torch.autograd.Function):
@@ -294,8 +305,8 @@ class _StridedWindowMatmulFunc(torch.autograd.Function):
         out = torch.empty((*dims, M, 2 * window_size + 1), dtype=inp.dtype, device=inp.device)
         if out.numel():
             x, y = _outer_addressable(inp, depth), _outer_addressable(other.transpose(-1, -2), depth)
-            g = N.geometry(_lead(inp[(0,) * depth]), M, Nh, window_size)
-            _outer_call(N.lib.wmm_band_nt_outer, depth, (x, y, out), (N.operand, N.operand, _pointer), g, N.dtype_code(inp))
+            g = N.geometry(_inner(inp, depth), M, Nh, window_size)
+            _outer_call(N.lib.wmm_band_nt_outer, depth, ((x, True), (y, True), (out, False)), g, N.dtype_code(inp))
         ctx.save_for_backward(inp, other)
         ctx.depth = depth
         return out
@@ -312,14 +323,13 @@ class _StridedWindowMatmulFunc(torch.autograd.Function):
         gkt = _grad_like(kt) if need[1] else None
         if inp.numel():
             x, y = _outer_addressable(inp, depth), _outer_addressable(kt, depth)
-            g, code = N.geometry(_lead(inp[(0,) * depth]), inp.shape[-2], inp.shape[-1], window_size), N.dtype_code(inp)
+            g, code = N.geometry(_inner(inp, depth), inp.shape[-2], inp.shape[-1], window_size), N.dtype_code(inp)
             if need[0] and need[1]:
-                _outer_call(N.lib.wmm_window_bwd_outer, depth, (x, y, grad_output, gq, gkt),
-                            (N.operand, N.operand, _pointer, N.operand, N.operand), g, code)
+                _outer_call(N.lib.wmm_window_bwd_outer, depth, ((x, True), (y, True), (grad_output, False), (gq, True), (gkt, True)), g, code)
             elif need[0]:
-                _outer_call(N.lib.wmm_band_n_outer, depth, (grad_output, y, gq), (_pointer, N.operand, N.operand), g, code)
+                _outer_call(N.lib.wmm_band_n_outer, depth, ((grad_output, False), (y, True), (gq, True)), g, code)
             elif need[1]:
-                _outer_call(N.lib.wmm_band_t_outer, depth, (grad_output, x, gkt), (_pointer, N.operand, N.operand), g, code)
+                _outer_call(N.lib.wmm_band_t_outer, depth, ((grad_output, False), (x, True), (gkt, True)), g, code)
         return gq, (gkt.transpose(-1, -2) if need[1] else None), None, None
 
 
@@ -333,8 +343,8 @@ class _StridedUnwindowMatmulFunc(torch.autograd.Function):
         out = torch.empty(other.shape, dtype=other.dtype, device=other.device)
         if out.numel():
             a, v = _outer_band(inp, depth), _outer_addressable(other, depth)
-            g = N.geometry(_lead(other[(0,) * depth]), other.shape[-2], other.shape[-1], window_size)
-            _outer_call(N.lib.wmm_band_n_outer, depth, (a, v, out), (_pointer, N.operand, N.operand), g, N.dtype_code(other))
+            g = N.geometry(_inner(other, depth), other.shape[-2], other.shape[-1], window_size)
+            _outer_call(N.lib.wmm_band_n_outer, depth, ((a, False), (v, True), (out, True)), g, N.dtype_code(other))
         ctx.save_for_backward(inp, other)
         ctx.depth = depth
         return out
@@ -349,24 +359,26 @@ class _StridedUnwindowMatmulFunc(torch.autograd.Function):
         gv = _grad_like(other) if need[1] else None
         if other.numel():
             v, go = _outer_addressable(other, depth), _outer_addressable(grad_output, depth)
-            g, code = N.geometry(_lead(other[(0,) * depth]), other.shape[-2], other.shape[-1], window_size), N.dtype_code(other)
+            g, code = N.geometry(_inner(other, depth), other.shape[-2], other.shape[-1], window_size), N.dtype_code(other)
             if need[0] and need[1]:
-                _outer_call(N.lib.wmm_unwindow_bwd_outer, depth, (_outer_band(inp, depth), v, go, ga, gv),
-                            (_pointer, N.operand, N.operand, _pointer, N.operand), g, code)
+                _outer_call(N.lib.wmm_unwindow_bwd_outer, depth, ((_outer_band(inp, depth), False), (v, True), (go, True), (ga, False), (gv, True)), g, code)
             elif need[0]:
-                _outer_call(N.lib.wmm_band_nt_outer, depth, (go, v, ga), (N.operand, N.operand, _pointer), g, code)
+                _outer_call(N.lib.wmm_band_nt_outer, depth, ((go, True), (v, True), (ga, False)), g, code)
             elif need[1]:
-                _outer_call(N.lib.wmm_band_t_outer, depth, (_outer_band(inp, depth), go, gv), (_pointer, N.operand, N.operand), g, code)
+                _outer_call(N.lib.wmm_band_t_outer, depth, ((_outer_band(inp, depth), False), (go, True), (gv, True)), g, code)
         return ga, gv, None, None
 
 
-def _pointer(t: torch.Tensor) -> int:
-    return t.data_ptr()
+def _inner(t: torch.Tensor, depth: int) -> int:
+    n = 1
+    for d in t.shape[depth:-2]:
+        n *= d
+    return n
 
 
 def _outer_band(t: torch.Tensor, depth: int) -> torch.Tensor:
     """A band whose slices below `depth` are contiguous."""
-    return t if t[(0,) * depth].is_contiguous() else t.contiguous()
+    return t if t.is_contiguous() or t[(0,) * depth].is_contiguous() else t.contiguous()
 
 
 # ---- autograd nodes and the public functions ------------------------------------------------------
