@@ -122,6 +122,17 @@ band_mm_tc_kernel(const __grid_constant__ CUtensorMap map_band, const __grid_con
     return t0 >= p.lo && t0 + 128 <= p.hi;
   };
 
+  // Chunks [c0, c1) of a tile: those whose positions (band_n) or band rows (band_t) meet the sequence; the others would be
+  // read from memory only to be zeroed.  (At least one, so that a tile outside the sequence is written as zeros.)  At both
+  // ends of a sequence a tile loses up to w / 128 chunks (B=96, M=4096, w=256: 6 of 160 chunks a sequence), and a window wider
+  // than the sequence costs what the sequence does (188 x 64 rows, N=64, w=256: 15 -> 5 us).
+  auto chunk_range = [&](bool tr, int t0, int &c0, int &c1) {
+    const int first = tr ? t0 - p.off - p.w : t0 - p.w + p.off;      // reduction index 0 of the tile
+    const int lo = tr ? 0 : p.lo, hi = tr ? p.M : p.hi;
+    c0 = min(max(lo - first, 0) >> 7, p.nchunks - 1);
+    c1 = max(c0 + 1, min(p.nchunks, (max(hi - first, 0) + 127) >> 7));
+  };
+
   // The MMA thread waits for the mask warps only at SYNC POINTS: every chunk that needs zeroing, and any
   // chunk that would otherwise be the STAGES-th in a row without one.  Both sides evaluate this rule on the
   // same chunk sequence.  Between two sync points fewer than STAGES chunks pass, so the producer can never
@@ -145,7 +156,9 @@ band_mm_tc_kernel(const __grid_constant__ CUtensorMap map_band, const __grid_con
         const bool tr = item_tr(wi);
         const CUtensorMap *map_other = (MODE == 2 && tr) ? &map_other1 : &map_other0;
         const int b = tile / p.tiles_per_batch, t0 = (tile % p.tiles_per_batch) * TILE;
-        for (int c = 0; c < p.nchunks; ++c, ++it) {
+        int c0, c1;
+        chunk_range(tr, t0, c0, c1);
+        for (int c = c0; c < c1; ++c, ++it) {
           const int s = it % S::STAGES;
           if (!(ok = mbar_wait(bar_empty(s), ((it / S::STAGES) & 1) ^ 1, abort_flag))) break;
           mbar_expect_tx(bar_full(s), S::STAGE_BYTES);
@@ -196,7 +209,9 @@ band_mm_tc_kernel(const __grid_constant__ CUtensorMap map_band, const __grid_con
         const uint64_t adesc = tr ? ADESC_T : ADESC_N;
         const int as = tit & 1;
         if (!(ok = mbar_wait(bar_acc_empty(as), ((tit >> 1) & 1) ^ 1, abort_flag))) break;
-        for (int c = 0; c < p.nchunks; ++c, ++it) {
+        int c0, c1;
+        chunk_range(tr, t0, c0, c1);
+        for (int c = c0; c < c1; ++c, ++it) {
           const int s = it % S::STAGES;
           // full: the TMA bytes have landed.  masked: the mask warps are done with this stage; waited for
           // only at sync points (see mask_sync below), i.e. for the chunks they had to touch.
@@ -212,7 +227,7 @@ band_mm_tc_kernel(const __grid_constant__ CUtensorMap map_band, const __grid_con
             const uint32_t a_off = tr ? (uint32_t)k * 2048u : BT::kstep_offset(k);
             const uint32_t b_off = ymn ? (uint32_t)(k >> 2) * (OT::BYTES / 2) + (uint32_t)(k & 3) * 32u : (uint32_t)k * 16u * OT::SW_BYTES;
             umma_f16(tmem_base + as * NH, smem_desc(adesc, a_addr + a_off), smem_desc(bdesc, b_addr + b_off), idesc,
-                     (c > 0 || k > 0) ? 1u : 0u);
+                     (c > c0 || k > 0) ? 1u : 0u);
           }
           umma_commit(bar_empty(s));
         }
@@ -228,7 +243,9 @@ band_mm_tc_kernel(const __grid_constant__ CUtensorMap map_band, const __grid_con
       const int tile = item_tile(wi);
       const bool tr = item_tr(wi);
       const int t0 = (tile % p.tiles_per_batch) * TILE;
-      for (int c = 0; c < p.nchunks; ++c, ++it) {
+      int c0, c1;
+      chunk_range(tr, t0, c0, c1);
+      for (int c = c0; c < c1; ++c, ++it) {
         const int s = it % S::STAGES;
         // every phase of every stage is observed (a parity wait cannot tell phases two apart)
         if (!(ok = mbar_wait(bar_full(s), (it / S::STAGES) & 1, abort_flag))) break;
