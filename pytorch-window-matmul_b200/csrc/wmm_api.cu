@@ -423,7 +423,7 @@ int wmm_band_t_edges(const void *band, const wmm_operand *x, const wmm_operand *
   if (edge_rows < 1 || 2 * (int64_t)edge_rows > g->other_rows || edge_skip < 0 || edge_skip >= edge_rows)
     return fail(WMM_ERR_SHAPE, "Input mismatch: %d edge rows (the outer %d skipped) at each end do not fit %d output rows",
                 edge_rows, edge_skip, g->other_rows);
-  if ((dtype != WMM_F16 && dtype != WMM_BF16) || pick_family(wmm::BAND_T, p) != 1)
+  if ((dtype != WMM_F16 && dtype != WMM_BF16) || (p.N != 32 && p.N != 64 && p.N != 128) || pick_family(wmm::BAND_T, p) != 1)
     return fail(WMM_ERR_UNSUPPORTED, "only the tensor-core band_t of the 16-bit types writes edge rows");
   p.edges = edges;
   p.edge_rows = edge_rows;

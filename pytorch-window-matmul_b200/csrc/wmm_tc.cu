@@ -220,6 +220,13 @@ cudaError_t launch_pdl(void (*kern)(KArgs...), int grid, int block, size_t smem,
   return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
 
+// The kernels are compiled for 32, 64 and 128 hidden columns.  A 16-bit problem with another multiple of 8 takes the next of them:
+// its tensor maps end at the true width, so loads fill the columns past it with zeros and stores leave them out.  The kernels are
+// bound by the band's bytes, which the padding does not touch.  Measured against the thread-fed kernels (wmm_tc_ragged.cuh), us:
+// fp16 64 x 4000, N = 48, w = 256: band_nt 98 -> 58, band_n 103 -> 58, band_t 106 -> 56, window backward 209 -> 104;
+// 3 x 25344, N = 120, w = 256: 50 -> 30, 40 -> 29, 40 -> 24, 81 -> 47.  (One loss seen: 400 x 128, N = 96, w = 40, band_n 10.8 -> 14.2.)
+int kernel_cols(int N) { return N <= 32 ? 32 : N <= 64 ? 64 : 128; }
+
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 CUtensorMapSwizzle swizzle_for(int bytes) {
@@ -249,12 +256,12 @@ bool make_operand_map(CUtensorMap *m, int et, const void *data, int cols, int ro
 }
 
 // 3-D map (positions, hidden, batch) over a 16-bit operand stored with the positions contiguous
-// (element (b, p, h) at b*stride_b + h*stride_c + p); box = (64 positions x `cols` hidden rows x 1), 128-byte swizzle.
-bool make_operand_map_mn(CUtensorMap *m, bool bf16, const void *data, int cols, int rows, int batch, int64_t stride_c,
+// (element (b, p, h) at b*stride_b + h*stride_c + p); box = (64 positions x `box_cols` hidden rows x 1), 128-byte swizzle.
+bool make_operand_map_mn(CUtensorMap *m, bool bf16, const void *data, int cols, int box_cols, int rows, int batch, int64_t stride_c,
                          int64_t stride_b) {
   const cuuint64_t dims[3] = {(cuuint64_t)rows, (cuuint64_t)cols, (cuuint64_t)batch};
   const cuuint64_t strides[2] = {(cuuint64_t)stride_c * 2, (cuuint64_t)(batch > 1 ? stride_b : (int64_t)cols * stride_c) * 2};
-  const cuuint32_t box[3] = {64, (cuuint32_t)cols, 1};
+  const cuuint32_t box[3] = {64, (cuuint32_t)box_cols, 1};
   const cuuint32_t estr[3] = {1, 1, 1};
   const CUresult r = encode_fn()(m, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3,
                                 const_cast<void *>(data), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -325,9 +332,9 @@ template <int ET, int NH, bool YMN, bool PAIRED> cudaError_t launch_nt(const Pro
   // The runtime call above has bound this thread to the device's primary context; the driver entry point
   // used for the tensor maps needs a current context (a fresh thread, e.g. an autograd worker, has none).
   CUtensorMap mx, my, mb;
-  if (!make_operand_map(&mx, BF16, p.a, NH, p.M, p.B, p.a_sr, p.a_sb, OT::BOXK) ||
-      !(YMN ? make_operand_map_mn(&my, BF16, p.b, NH, p.Mo, p.B, p.b_sc, p.b_sb)
-            : make_operand_map(&my, BF16, p.b, NH, p.Mo, p.B, p.b_sr, p.b_sb, OT::BOXK)) ||
+  if (!make_operand_map(&mx, BF16, p.a, p.N, p.M, p.B, p.a_sr, p.a_sb, OT::BOXK) ||
+      !(YMN ? make_operand_map_mn(&my, BF16, p.b, p.N, NH, p.Mo, p.B, p.b_sc, p.b_sb)
+            : make_operand_map(&my, BF16, p.b, p.N, p.Mo, p.B, p.b_sr, p.b_sb, OT::BOXK)) ||
       !make_band_map(&mb, BF16, p.o, p.M, p.w, p.B, p.band_sb))
     return cudaErrorInvalidValue;
   const int grid = persistent_grid(k.total_tiles);
@@ -376,13 +383,13 @@ template <bool BF16, int NH, int MODE, bool YMN> cudaError_t launch_mm(const Pro
   // (the tensor maps need the current context the runtime call above has bound to this thread)
   CUtensorMap mband, mother0, mout0, mother1, mout1;
   if (!make_band_map(&mband, BF16, p.a, p.M, p.w, p.B, p.band_sb) ||
-      !(YMN ? make_operand_map_mn(&mother0, BF16, p.b, NH, other_rows, p.B, p.b_sc, p.b_sb)
-            : make_operand_map(&mother0, BF16, p.b, NH, other_rows, p.B, p.b_sr, p.b_sb, OT::BOXK)) ||
-      !make_operand_map(&mout0, BF16, p.o, NH, out_rows, p.B, p.o_sr, p.o_sb, OT::BOXK))
+      !(YMN ? make_operand_map_mn(&mother0, BF16, p.b, p.N, NH, other_rows, p.B, p.b_sc, p.b_sb)
+            : make_operand_map(&mother0, BF16, p.b, p.N, other_rows, p.B, p.b_sr, p.b_sb, OT::BOXK)) ||
+      !make_operand_map(&mout0, BF16, p.o, p.N, out_rows, p.B, p.o_sr, p.o_sb, OT::BOXK))
     return cudaErrorInvalidValue;
   if (MODE == 2) {
-    if (!make_operand_map(&mother1, BF16, pt->b, NH, pt->M, pt->B, pt->b_sr, pt->b_sb, OT::BOXK) ||
-        !make_operand_map(&mout1, BF16, pt->o, NH, pt->Mo, pt->B, pt->o_sr, pt->o_sb, OT::BOXK))
+    if (!make_operand_map(&mother1, BF16, pt->b, pt->N, pt->M, pt->B, pt->b_sr, pt->b_sb, OT::BOXK) ||
+        !make_operand_map(&mout1, BF16, pt->o, pt->N, pt->Mo, pt->B, pt->o_sr, pt->o_sb, OT::BOXK))
       return cudaErrorInvalidValue;
   } else {
     mother1 = mother0;
@@ -397,7 +404,7 @@ template <bool BF16, int NH, int MODE, bool YMN> cudaError_t launch_mm(const Pro
 
 template <int MODE, bool YMN> cudaError_t launch_mm_n(const Problem &p, const Problem *pt, cudaStream_t stream) {
   const bool bf16 = p.dtype == WMM_BF16;
-  switch (p.N) {
+  switch (kernel_cols(p.N)) {
     case 32: return bf16 ? launch_mm<true, 32, MODE, YMN>(p, pt, stream) : launch_mm<false, 32, MODE, YMN>(p, pt, stream);
     case 64: return bf16 ? launch_mm<true, 64, MODE, YMN>(p, pt, stream) : launch_mm<false, 64, MODE, YMN>(p, pt, stream);
     case 128: return bf16 ? launch_mm<true, 128, MODE, YMN>(p, pt, stream) : launch_mm<false, 128, MODE, YMN>(p, pt, stream);
@@ -445,6 +452,7 @@ bool sweep_eligible(const Problem &pn, const Problem &pt) {
   const int D = pn.w / 128;
   if (2 * D + 2 > SweepSmem<32>::MAX_SLOTS || (2 * D + 4) * pn.N > 512) return false;
   if (pn.lo != 0 || pn.hi != pn.M || y_position_major(pn)) return false;
+  if (pn.N != kernel_cols(pn.N)) return false;   // (the sweep stores whole accumulator rows)
   // A run that starts inside a sequence replays D (2D + 1) boxes; with short runs (few row tiles per CTA) that costs
   // more than the second pass of the two-pass kernel.
   const int64_t row_tiles = (int64_t)pn.B * ((pn.M + TILE - 1) / TILE);
@@ -544,6 +552,11 @@ template <bool BF16, int NH> cudaError_t launch_ragged_nh(Primitive prim, const 
 
 }  // namespace
 
+// Hidden sizes that are no kernel width.  (WMM_FLAG_REQUIRE_TENSOR and a band with a batch stride keep to the widths proper.)
+static bool padded_cols_ok(Primitive prim, const Problem &p) {
+  return p.N >= 8 && p.N <= 128 && (p.N % 8) == 0 && !(p.flags & WMM_FLAG_REQUIRE_TENSOR) && p.band_sb == (int64_t)p.M * (2ll * p.w + 1);
+}
+
 bool tensor_eligible(Primitive prim, const Problem &p) {
   if (p.dtype == WMM_F32) {
     // fp32 operands go to the tensor cores only on request (WMM_FLAG_TF32: products of tf32-rounded values, fp32 sums)
@@ -563,7 +576,7 @@ bool tensor_eligible(Primitive prim, const Problem &p) {
   }
   if (p.dtype != WMM_F16 && p.dtype != WMM_BF16) return false;
   if (!encode_fn()) return false;
-  if (p.N != 32 && p.N != 64 && p.N != 128) return false;
+  if (p.N != 32 && p.N != 64 && p.N != 128 && !padded_cols_ok(prim, p)) return false;
   if ((int64_t)p.B * ((p.M + TILE - 1) / TILE) > 0x7fffffffLL) return false;
   switch (prim) {
     case BAND_NT:
@@ -584,7 +597,7 @@ bool tensor_eligible(Primitive prim, const Problem &p) {
 cudaError_t launch_tensor(Primitive prim, const Problem &p, cudaStream_t stream, int *launches) {
   cudaError_t e = cudaErrorNotSupported;
   if (prim == BAND_NT) {
-    switch (p.N) {
+    switch (kernel_cols(p.N)) {   // (fp32 problems have 32 or 64)
       case 32: e = launch_nt_any<32>(p, stream); break;
       case 64: e = launch_nt_any<64>(p, stream); break;
       case 128: e = launch_nt_any<128>(p, stream); break;
