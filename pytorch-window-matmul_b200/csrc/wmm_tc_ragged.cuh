@@ -131,11 +131,31 @@ template <int LINES>
 __device__ __forceinline__ void load_position_lines(const uint16_t *base, int64_t sc, int N, int h0, int64_t first, int64_t lo, int64_t hi,
                                                     uint32_t tile, int lane) {
   const int e0 = (int)max((int64_t)0, min((int64_t)64, lo - first)), e1 = (int)max((int64_t)0, min((int64_t)64, hi - first));
+  // With the elements before and after the line in the sequence too, a line at an odd element is put together from the words
+  // around it (two loads, one shift) instead of single elements, whose two predicated loads each waited for the one before.
+  const bool words = first > lo && first + 65 <= hi;
 #pragma unroll 1
   for (int q = 0; q < LINES; q += 8) {
     uint32_t v[8];
+    if (words) {
+      uint32_t next[8];
 #pragma unroll
-    for (int u = 0; u < 8; u++) v[u] = h0 + q + u < N ? line_pair(base + (h0 + q + u) * sc + first, lane, e0, e1) : 0u;
+      for (int u = 0; u < 8; u++) {
+        const uintptr_t at = reinterpret_cast<uintptr_t>(base + (h0 + q + u) * sc + first);
+        const uint32_t *src = reinterpret_cast<const uint32_t *>(at & ~(uintptr_t)3) + lane;
+        v[u] = next[u] = 0;
+        if (h0 + q + u < N) {
+          v[u] = src[0];
+          if (at & 2) next[u] = src[1];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 8; u++)
+        if (reinterpret_cast<uintptr_t>(base + (h0 + q + u) * sc + first) & 2) v[u] = __funnelshift_r(v[u], next[u], 16);
+    } else {
+#pragma unroll
+      for (int u = 0; u < 8; u++) v[u] = h0 + q + u < N ? line_pair(base + (h0 + q + u) * sc + first, lane, e0, e1) : 0u;
+    }
 #pragma unroll
     for (int u = 0; u < 8; u++) sts32(rag_word(tile, h0 + q + u, lane), v[u]);
   }
